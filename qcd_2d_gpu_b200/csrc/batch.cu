@@ -167,13 +167,13 @@ __global__ void __launch_bounds__(kBlock) batch_normalize(BatchView B) {
 // CTA adds their partials in the same order, so every replica's numbers are
 // those of the same lattice measured alone, bit for bit.
 template <bool FP64>
-__global__ void __launch_bounds__(kBlock) batch_measure(BatchView B, double2* partials, unsigned int* rep_count,
+__global__ void __launch_bounds__(kBlock, FP64 ? kMeasurePerSM64 : kMeasurePerSM32) batch_measure(BatchView B, double2* partials, unsigned int* rep_count,
                                                         unsigned int* all_count, int* cursor, double2* series,
                                                         int cap) {
   const int mcta = (int)blockIdx.x + B.mcta0;  // CTA in the batch's measurement table
   const int r = __ldg(B.mcta_rep + mcta);
   const Replica& R = B.rep[r];
-  const int nblk = (int)measure_blocks(R.g.vh);
+  const int nblk = (int)measure_blocks(R.g.vh, FP64 ? kMeasurePerSM64 : kMeasurePerSM32);
   const int k = *(volatile int*)cursor;  // advanced only by the last CTA below
   double e = 0, pl = 0;
   if (FP64) {
@@ -511,7 +511,7 @@ int qcd_batch_create(const qcd_replica* r, int n, const qcd_params* common, qcd_
     rng_off += 6 * (V / 2);
     site_off += V;
     cta += (int)((V / 2 + kBlock - 1) / kBlock);
-    mcta += (int)measure_blocks(V / 2);
+    mcta += (int)measure_blocks(V / 2, common->precision == QCD_PREC_FP64 ? kMeasurePerSM64 : kMeasurePerSM32);
   }
   b->sites = site_off;
   b->ctas = cta;

@@ -164,22 +164,22 @@ __global__ void __launch_bounds__(kBlock) soa_to_aos32(Links32 L, double* __rest
 // en_av<PMC> (observables.h:99-141): energy = mean of -(1 - P_xt), plaquette
 // = mean of (P_yx + P_yt + P_xt)/3; with PMC the y plaquettes at y = Ly-1 count
 // as 1.  out[0] = energy, out[1] = plaquette.
-template <class L, int PMC>
-__global__ void __launch_bounds__(kBlock) measure(L links, Geo g, double2* partials,
-                                                  unsigned int* counter, double* out) {
+template <class L, int PMC, int PER_SM>
+__global__ void __launch_bounds__(kBlock, PER_SM) measure(L links, Geo g, double2* partials, unsigned int* counter,
+                                                          double* out, const int* err) {
   double e = 0, pl = 0;
-  measure_sites<L, PMC != 0>(links, g, blockIdx.x, gridDim.x, e, pl);  // grid: measure_blocks(V/2)
+  measure_sites<L, PMC != 0>(links, g, blockIdx.x, gridDim.x, e, pl);  // grid: measure_blocks(V/2, PER_SM)
   double se, sp;
   block_sum2(e, pl * (1.0 / 3.0), &se, &sp);
   if (threadIdx.x == 0) partials[blockIdx.x] = make_double2(se, sp);
-  finish_sum2(partials, counter, 1.0 / (2.0 * (double)g.vh), out);
+  finish_sum2(partials, counter, 1.0 / (2.0 * (double)g.vh), out, err);
 }
 
 // Unitarity: out[0] = mean det, out[1] = number of links with |det-1| > tol
 // or not finite (print_det, lattice_setup.h:176-183, plus a NaN/Inf check).
 template <class L>
 __global__ void __launch_bounds__(kBlock) unitarity(L links, int vh, double tol, double2* partials,
-                                                    unsigned int* counter, double* out) {
+                                                    unsigned int* counter, double* out, const int* err) {
   const int id = blockIdx.x * kBlock + threadIdx.x;
   double s = 0, bad = 0;
   if (id < vh) {
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kBlock) unitarity(L links, int vh, double tol,
   double ss, sb;
   block_sum2(s, bad, &ss, &sb);
   if (threadIdx.x == 0) partials[blockIdx.x] = make_double2(ss, sb);
-  finish_sum2(partials, counter, 1.0, out);
+  finish_sum2(partials, counter, 1.0, out, err);
 }
 
 // ----------------------------------------------------------- RNG tape ----

@@ -267,16 +267,16 @@ __device__ __forceinline__ float2 plaq2(const Pair32& P, int mu, int nu, int p, 
   return p2_retr_bd(B, P.ld(nu, p, id));
 }
 
-// Items k = c*256 + tid, + nb*256, ... below 2 V/4: pair k - p V/4 of
-// sublattice p = k / (V/4), both lanes; deterministic per-CTA partials as
-// in measure (kernels.cuh).
+// The sums of CTA c of nb as in measure_sites, a pair of sites per thread and
+// turn; deterministic per-CTA partials as in measure (kernels.cuh).
 template <bool PMC>
 __device__ __forceinline__ void measure_pairs(const Pair32& P, const Geo& gh, int c, int nb, double& e, double& pl) {
-  const unsigned int items = 2u * (unsigned int)gh.vh;
-  for (unsigned int k = (unsigned int)c * kBlock + threadIdx.x; k < items; k += (unsigned int)nb * kBlock) {
-    const int p = k >= (unsigned int)gh.vh;
-    const int id = (int)k - p * gh.vh;
-    const int r = div_by((unsigned int)id, gh.slice_m);
+  const int p = threadIdx.x >= kMeasureIds;
+  const unsigned int pairs = (unsigned int)gh.vh;
+  for (unsigned int k = (unsigned int)c * kMeasureIds + threadIdx.x % kMeasureIds; k < pairs;
+       k += (unsigned int)nb * kMeasureIds) {
+    const int id = (int)k;
+    const int r = div_by(k, gh.slice_m);
     const int s = id - r * gh.slice;
     const Nbr n = make_nbr_slice(gh, s, r, p);
     const bool sp = r == gh.lt - 1;
@@ -295,14 +295,15 @@ __device__ __forceinline__ void measure_pairs(const Pair32& P, const Geo& gh, in
 }
 
 template <int PMC>
-__global__ void __launch_bounds__(kBlock) measure_p(Pair32 P, Geo gh, double2* partials, unsigned int* counter,
-                                                    double* out) {
+__global__ void __launch_bounds__(kBlock, kMeasurePerSMPair) measure_p(Pair32 P, Geo gh, double2* partials,
+                                                                       unsigned int* counter, double* out,
+                                                                       const int* err) {
   double e = 0, pl = 0;
-  measure_pairs<PMC != 0>(P, gh, blockIdx.x, gridDim.x, e, pl);  // grid: measure_blocks(V/2)
+  measure_pairs<PMC != 0>(P, gh, blockIdx.x, gridDim.x, e, pl);  // grid: measure_blocks(V/4, kMeasurePerSMPair)
   double se, sp;
   block_sum2(e, pl * (1.0 / 3.0), &se, &sp);
   if (threadIdx.x == 0) partials[blockIdx.x] = make_double2(se, sp);
-  finish_sum2(partials, counter, 1.0 / (4.0 * (double)gh.vh), out);
+  finish_sum2(partials, counter, 1.0 / (4.0 * (double)gh.vh), out, err);
 }
 
 // ------------------------------------------------ whole-store kernels ----
@@ -321,7 +322,7 @@ static __global__ void __launch_bounds__(kBlock) normalize32p(Pair32 P) {
 
 // unitarity (kernels.cuh): thread per pair
 static __global__ void __launch_bounds__(kBlock) unitarity_p(Pair32 P, double tol, double2* partials, unsigned int* counter,
-                                                      double* out) {
+                                                      double* out, const int* err) {
   const int j = blockIdx.x * kBlock + threadIdx.x;
   double s = 0, bad = 0;
   if (j < P.vhp) {
@@ -339,7 +340,7 @@ static __global__ void __launch_bounds__(kBlock) unitarity_p(Pair32 P, double to
   double ss, sb;
   block_sum2(s, bad, &ss, &sb);
   if (threadIdx.x == 0) partials[blockIdx.x] = make_double2(ss, sb);
-  finish_sum2(partials, counter, 1.0, out);
+  finish_sum2(partials, counter, 1.0, out, err);
 }
 
 // reference AoS (phi[(p*Vh + id)*12 + d*4 + c]) <-> paired store, thread per site

@@ -46,8 +46,8 @@ struct qcd_lattice {
   // reductions
   double2* partials = nullptr;
   unsigned int* counter = nullptr;
-  double* result = nullptr;      // 2 doubles on the device
-  double* result_host = nullptr; // pinned
+  double* result_host = nullptr; // pinned: two sums, the error word, a word for copies
+  double* result_dev = nullptr;  // the same memory as the device addresses it
   int* err = nullptr;            // device error word
   // measurement series
   double* series = nullptr;
@@ -537,14 +537,7 @@ int pass_pairs(qcd_lattice* h, int kind, int renorm) {
   return QCD_OK;
 }
 
-int run_passes(qcd_lattice* h, const PassSpec* ps, int np);
-
-int check_device_error(qcd_lattice* h) {
-  int e = 0;
-  CUDA_OR_FAIL(h, cudaMemcpyAsync(&h->result_host[2], h->err, sizeof(int), cudaMemcpyDeviceToHost,
-                                  h->stream));
-  CUDA_OR_FAIL(h, cudaStreamSynchronize(h->stream));
-  memcpy(&e, &h->result_host[2], sizeof(int));
+int report_device_error(qcd_lattice* h, int e) {
   if (e & DEVERR_TIMEOUT) {
     CUDA_OR_FAIL(h, cudaMemsetAsync(h->err, 0, sizeof(int), h->stream));
     CUDA_OR_FAIL(h, cudaStreamSynchronize(h->stream));
@@ -558,34 +551,49 @@ int check_device_error(qcd_lattice* h) {
   return QCD_OK;
 }
 
+int check_device_error(qcd_lattice* h) {
+  int e = 0;
+  CUDA_OR_FAIL(h, cudaMemcpyAsync(&h->result_host[2], h->err, sizeof(int), cudaMemcpyDeviceToHost,
+                                  h->stream));
+  CUDA_OR_FAIL(h, cudaStreamSynchronize(h->stream));
+  memcpy(&e, &h->result_host[2], sizeof(int));
+  return report_device_error(h, e);
+}
+
+// The answer of a reduction launched with result_dev and the error word: the
+// kernel itself has written both to the pinned result_host.
 int reduce_result(qcd_lattice* h, double* a, double* b) {
-  CUDA_OR_FAIL(h, cudaMemcpyAsync(h->result_host, h->result, 2 * sizeof(double),
-                                  cudaMemcpyDeviceToHost, h->stream));
-  int rc = check_device_error(h);  // synchronises the stream
+  int e = 0;
+  CUDA_OR_FAIL(h, cudaStreamSynchronize(h->stream));
+  memcpy(&e, &h->result_host[2], sizeof(int));
+  int rc = report_device_error(h, e);
   if (rc) return rc;
   if (a) *a = h->result_host[0];
   if (b) *b = h->result_host[1];
   return QCD_OK;
 }
 
-int launch_measure(qcd_lattice* h, double* out_dev) {
-  const unsigned int nb = measure_blocks(h->g.vh);
+// `err`: the device error word where out_dev has room for it (finish_sum2), or null
+int launch_measure(qcd_lattice* h, double* out_dev, const int* err) {
   const bool pmc = h->p.boundary == QCD_BC_PMC;
   if (h->p.precision == QCD_PREC_FP64) {
+    const unsigned int nb = measure_blocks(h->g.vh, kMeasurePerSM64);
     if (pmc)
-      measure<Links64, 1><<<nb, kBlock, 0, h->stream>>>(links64(h), h->g, h->partials, h->counter, out_dev);
+      measure<Links64, 1, kMeasurePerSM64><<<nb, kBlock, 0, h->stream>>>(links64(h), h->g, h->partials, h->counter, out_dev, err);
     else
-      measure<Links64, 0><<<nb, kBlock, 0, h->stream>>>(links64(h), h->g, h->partials, h->counter, out_dev);
+      measure<Links64, 0, kMeasurePerSM64><<<nb, kBlock, 0, h->stream>>>(links64(h), h->g, h->partials, h->counter, out_dev, err);
   } else if (h->paired) {
+    const unsigned int nb = measure_blocks(h->gh.vh, kMeasurePerSMPair);
     if (pmc)
-      measure_p<1><<<nb, kBlock, 0, h->stream>>>(pair32(h), h->gh, h->partials, h->counter, out_dev);
+      measure_p<1><<<nb, kBlock, 0, h->stream>>>(pair32(h), h->gh, h->partials, h->counter, out_dev, err);
     else
-      measure_p<0><<<nb, kBlock, 0, h->stream>>>(pair32(h), h->gh, h->partials, h->counter, out_dev);
+      measure_p<0><<<nb, kBlock, 0, h->stream>>>(pair32(h), h->gh, h->partials, h->counter, out_dev, err);
   } else {
+    const unsigned int nb = measure_blocks(h->g.vh, kMeasurePerSM32);
     if (pmc)
-      measure<Links32, 1><<<nb, kBlock, 0, h->stream>>>(links32(h), h->g, h->partials, h->counter, out_dev);
+      measure<Links32, 1, kMeasurePerSM32><<<nb, kBlock, 0, h->stream>>>(links32(h), h->g, h->partials, h->counter, out_dev, err);
     else
-      measure<Links32, 0><<<nb, kBlock, 0, h->stream>>>(links32(h), h->g, h->partials, h->counter, out_dev);
+      measure<Links32, 0, kMeasurePerSM32><<<nb, kBlock, 0, h->stream>>>(links32(h), h->g, h->partials, h->counter, out_dev, err);
   }
   LAUNCH_CHECK(h);
   return QCD_OK;
@@ -644,7 +652,6 @@ void release(qcd_lattice* h) {
   cudaFree(h->accept);
   cudaFree(h->partials);
   cudaFree(h->counter);
-  cudaFree(h->result);
   cudaFree(h->err);
   cudaFree(h->draw_dev);
   cudaFree(h->series);
@@ -740,14 +747,15 @@ int qcd_create(const qcd_params* p, qcd_lattice** out) {
     step(cudaMalloc(&h->accept, 2 * vh * sizeof(int)), "cudaMalloc(accept)");
     if (rc == QCD_OK) step(cudaMemsetAsync(h->accept, 0, 2 * vh * sizeof(int), h->stream), "memset");
   }
-  const size_t nb = nblocks(h->g.vh);  // one partial per CTA of the largest reduction launch
+  // one partial per CTA of the largest reduction launch
+  const size_t nb = std::max(nblocks(h->g.vh), measure_blocks(h->g.vh, kMeasurePerSM32));
   if (rc == QCD_OK) step(cudaMalloc(&h->partials, nb * sizeof(double2)), "cudaMalloc(partials)");
   if (rc == QCD_OK) step(cudaMalloc(&h->counter, sizeof(unsigned int)), "cudaMalloc(counter)");
-  if (rc == QCD_OK) step(cudaMalloc(&h->result, 2 * sizeof(double)), "cudaMalloc(result)");
   if (rc == QCD_OK) step(cudaMalloc(&h->err, sizeof(int)), "cudaMalloc(err)");
   if (rc == QCD_OK) step(cudaMalloc(&h->draw_dev, sizeof(unsigned long long)), "cudaMalloc(draw counter)");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->draw_dev, 0, sizeof(unsigned long long), h->stream), "memset");
   if (rc == QCD_OK) step(cudaMallocHost(&h->result_host, 4 * sizeof(double)), "cudaMallocHost");
+  if (rc == QCD_OK) step(cudaHostGetDevicePointer((void**)&h->result_dev, h->result_host, 0), "cudaHostGetDevicePointer");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->counter, 0, sizeof(unsigned int), h->stream), "memset");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "memset");
   // the FP64 sweep draws from the stored MRG32k3a streams at every update; an
@@ -1150,7 +1158,7 @@ int qcd_wave_selftest_timeout(qcd_lattice* h) {
 
 int qcd_measure(qcd_lattice* h, double* energy, double* plaquette) {
   if (!h) return QCD_ERR_INVALID;
-  int rc = launch_measure(h, h->result);
+  int rc = launch_measure(h, h->result_dev, h->err);
   if (rc) return rc;
   return reduce_result(h, energy, plaquette);
 }
@@ -1171,7 +1179,7 @@ int qcd_series_reserve(qcd_lattice* h, int capacity) {
 int qcd_measure_into_series(qcd_lattice* h, int index) {
   if (!h || index < 0 || index >= h->series_cap)
     return fail(h, QCD_ERR_INVALID, "series index %d outside capacity %d", index, h ? h->series_cap : 0);
-  return launch_measure(h, h->series + 2 * (size_t)index);
+  return launch_measure(h, h->series + 2 * (size_t)index, nullptr);
 }
 
 int qcd_series_read(qcd_lattice* h, double* energy, double* plaquette, int n) {
@@ -1233,11 +1241,11 @@ int qcd_check_unitarity(qcd_lattice* h, double tol, double* mean_det) {
   if (!h || !(tol >= 0)) return QCD_ERR_INVALID;
   const unsigned int nb = nblocks(h->g.vh);
   if (h->p.precision == QCD_PREC_FP64)
-    unitarity<<<nb, kBlock, 0, h->stream>>>(links64(h), h->g.vh, tol, h->partials, h->counter, h->result);
+    unitarity<<<nb, kBlock, 0, h->stream>>>(links64(h), h->g.vh, tol, h->partials, h->counter, h->result_dev, h->err);
   else if (h->paired)
-    unitarity_p<<<nblocks(h->gh.vh), kBlock, 0, h->stream>>>(pair32(h), tol, h->partials, h->counter, h->result);
+    unitarity_p<<<nblocks(h->gh.vh), kBlock, 0, h->stream>>>(pair32(h), tol, h->partials, h->counter, h->result_dev, h->err);
   else
-    unitarity<<<nb, kBlock, 0, h->stream>>>(links32(h), h->g.vh, tol, h->partials, h->counter, h->result);
+    unitarity<<<nb, kBlock, 0, h->stream>>>(links32(h), h->g.vh, tol, h->partials, h->counter, h->result_dev, h->err);
   LAUNCH_CHECK(h);
   double sum = 0, bad = 0;
   int rc = reduce_result(h, &sum, &bad);
@@ -1353,7 +1361,7 @@ __device__ __forceinline__ Quat<double> ld64<LinksAoS>(const LinksAoS& links, in
 }  // namespace qcd
 
 // partial sums of at most QCD_NOALLOC_MAX_BLOCKS CTAs, then the arrival counter
-static_assert(kMeasureMaxBlocks <= QCD_NOALLOC_MAX_BLOCKS,
+static_assert(kMeasureSMs * kMeasurePerSM64 <= QCD_NOALLOC_MAX_BLOCKS,
               "a measurement may launch more CTAs than the no-allocation scratch has partial sums");
 static_assert((long long)QCD_NOALLOC_MAX_HALF_SITES * 6 < (1ll << 31), "32-bit plane indices");
 static constexpr size_t kNoAllocCounterOffset = (size_t)QCD_NOALLOC_MAX_BLOCKS * sizeof(double2);
@@ -1397,7 +1405,7 @@ extern "C" int qcd_measure_aos_noalloc(const double* phi_dev, int lt, int lx, in
     return QCD_ERR_UNSUPPORTED;
   }
   const long long vh = (long long)lt * lx * ly / 2;
-  if (measure_blocks(vh) > QCD_NOALLOC_MAX_BLOCKS) return QCD_ERR_UNSUPPORTED;  // excluded by the static_assert
+  if (measure_blocks(vh, kMeasurePerSM64) > QCD_NOALLOC_MAX_BLOCKS) return QCD_ERR_UNSUPPORTED;  // excluded by the static_assert
   void* base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc) return rc;
@@ -1409,11 +1417,11 @@ extern "C" int qcd_measure_aos_noalloc(const double* phi_dev, int lt, int lx, in
   if (e == cudaSuccess) {
     Geo g = make_geo(lt, lx, ly);
     LinksAoS L{phi_dev, (int)vh};
-    const unsigned int grid = measure_blocks(vh);  // the same grid, so the same sums, as qcd_measure
+    const unsigned int grid = measure_blocks(vh, kMeasurePerSM64);  // the same grid, so the same sums, as qcd_measure
     if (boundary == QCD_BC_PMC)
-      measure<LinksAoS, 1><<<grid, kBlock, 0, s>>>(L, g, partials, counter, out_dev);
+      measure<LinksAoS, 1, kMeasurePerSM64><<<grid, kBlock, 0, s>>>(L, g, partials, counter, out_dev, nullptr);
     else
-      measure<LinksAoS, 0><<<grid, kBlock, 0, s>>>(L, g, partials, counter, out_dev);
+      measure<LinksAoS, 0, kMeasurePerSM64><<<grid, kBlock, 0, s>>>(L, g, partials, counter, out_dev, nullptr);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

@@ -163,9 +163,11 @@ __device__ __forceinline__ void block_sum2(double v0, double v1, double* out0, d
 }
 
 // After thread 0 of every CTA stored its partial pair: the last CTA adds all
-// partials in order, scales them and writes out[0..1].
+// partials in order, scales them and writes out[0..1]; with `err` also the
+// device error word, as the int at out[2] (`out` is then the caller's pinned
+// host memory, and one kernel brings the whole answer).
 __device__ __forceinline__ void finish_sum2(double2* partials, unsigned int* counter, double scale,
-                                            double* out) {
+                                            double* out, const int* err = nullptr) {
   __shared__ bool last;
   const unsigned int ctas = gridDim.x;
   if (threadIdx.x == 0) {
@@ -189,6 +191,7 @@ __device__ __forceinline__ void finish_sum2(double2* partials, unsigned int* cou
   if (threadIdx.x == 0) {
     out[0] = sa * scale;
     out[1] = sb * scale;
+    if (err) *reinterpret_cast<int*>(out + 2) = __ldcg(err);
     *counter = 0u;
   }
 }
@@ -227,32 +230,44 @@ __device__ __forceinline__ double plaq(const L& links, int mu, int nu, int p, in
   return 1 - A.w;
 }
 
-// CTAs of a measurement: one per 1024 half-lattice sites (each thread then
-// sums at least four sites of each parity, which amortises the CTA's
-// reduction) up to a fixed cap, the threads striding over the sites, so a
-// large lattice makes a few thousand partial sums (added by the last CTA).
-// The count depends on the lattice only, so the summation order is the same
-// on every device and for a lattice measured alone or in a batch.
-constexpr long long kMeasureMaxBlocks = 4096;
-constexpr long long kMeasureSitesPerBlock = 4 * kBlock;
-__host__ __device__ __forceinline__ unsigned int measure_blocks(long long vh) {
-  const long long nb = (vh + kMeasureSitesPerBlock - 1) / kMeasureSitesPerBlock;
-  return (unsigned int)(nb < kMeasureMaxBlocks ? nb : kMeasureMaxBlocks);
+// A measurement covers kMeasureIds sublattice indices of both parities per CTA
+// and turn: warps 0-3 take the even sites, warps 4-7 the odd sites of the same
+// indices.  The two need the same six link classes (a site's own links are the
+// other's neighbours), so each link leaves HBM once; taking all even sites
+// before all odd ones read the store twice.
+//
+// Bound by HBM on a large lattice, by the latency of one turn on a small one.
+// A small lattice gets a CTA per 128 indices, one turn each, as long as that
+// leaves SMs idle (16^3: 7 us; with eight sites in series per thread 14 us);
+// above, four turns per CTA, which amortise its reduction where other launches
+// fill the GPU (a batch of 96 replicas: 3% of its run).  A large one gets the CTAs that are
+// resident at once on 148 SMs at the kernel's register count, which then walk
+// the lattice side by side, so neighbours meet in L1 and L2 and no last wave
+// runs half empty.  384^3: FP64 0.95 ms at 2 CTAs per SM (1.26 ms with twice as
+// many CTAs, 1.7 ms with a CTA per 1024 indices and one parity after the other),
+// FP32 0.55 ms at 4, site pairs 0.48 ms at 3 (0.89 ms before).
+constexpr int kMeasureIds = kBlock / 2;
+constexpr int kMeasureSMs = 148;
+constexpr int kMeasurePerSM64 = 2, kMeasurePerSM32 = 4, kMeasurePerSMPair = 3;
+// CTAs of a measurement over `ids` sublattice indices (pairs of them in the
+// site-pair store).  The count depends on the lattice only, so the summation
+// order is the same on every device and for a lattice measured alone or in a batch.
+__host__ __device__ __forceinline__ unsigned int measure_blocks(long long ids, int per_sm) {
+  const long long one = (ids + kMeasureIds - 1) / kMeasureIds, four = (one + 3) / 4;
+  const long long most = one < kMeasureSMs ? one : four > kMeasureSMs ? four : kMeasureSMs;
+  return (unsigned int)(most < kMeasureSMs * per_sm ? most : kMeasureSMs * per_sm);
 }
 
-// Energy and plaquette sums of the items k = c*256 + tid, + nb*256, ... of
-// CTA c of nb, item k < V being the site of sublattice p = k / (V/2) with
-// sublattice index k - p V/2: -(1 - P_xt) and 3 - the sum of the three 1 - P.
-// One site of one parity per item keeps few links live per thread.  A
-// multiply-high finds the site's t-slice; the neighbours come from the slice
-// position (multiply-high).
+// Energy and plaquette sums of CTA c of nb: -(1 - P_xt) and 3 - the sum of the
+// three 1 - P of each site.  One site per thread and turn keeps few links live.
 template <class L, bool PMC>
 __device__ __forceinline__ void measure_sites(const L& links, const Geo& g, int c, int nb, double& e, double& pl) {
-  const unsigned int items = 2u * (unsigned int)g.vh;
-  for (unsigned int k = (unsigned int)c * kBlock + threadIdx.x; k < items; k += (unsigned int)nb * kBlock) {
-    const int p = k >= (unsigned int)g.vh;
-    const int id = (int)k - p * g.vh;
-    const int t = div_by((unsigned int)id, g.slice_m);
+  const int p = threadIdx.x >= kMeasureIds;
+  const unsigned int ids = (unsigned int)g.vh;
+  for (unsigned int k = (unsigned int)c * kMeasureIds + threadIdx.x % kMeasureIds; k < ids;
+       k += (unsigned int)nb * kMeasureIds) {
+    const int id = (int)k;
+    const int t = div_by(k, g.slice_m);
     const int s = id - t * g.slice;
     const Nbr n = make_nbr_slice(g, s, t, p);
     double a = plaq(links, DIR_Y, DIR_X, p, id, n.yp, n.xp);
