@@ -824,24 +824,26 @@ static int ensure_stage(qcd_lattice* h) {
 
 int qcd_load_config_device(qcd_lattice* h, const double* aos_dev) {
   if (!h || !aos_dev) return QCD_ERR_INVALID;
+  const dim3 grid(nblocks(h->g.vh), 2), grid_p((unsigned int)((h->gh.vh + kAosPairs - 1) / kAosPairs), 2);
   if (h->p.precision == QCD_PREC_FP64)
-    aos_to_soa64<<<nblocks(h->g.vh), kBlock, 0, h->stream>>>(aos_dev, links64(h), h->g.vh);
+    aos_to_soa<<<grid, kBlock, 0, h->stream>>>(aos_dev, links64(h), h->g.vh);
   else if (h->paired)
-    aos_to_pair32<<<nblocks(h->g.vh), kBlock, 0, h->stream>>>(aos_dev, pair32(h), h->g.vh);
+    aos_to_pair32<<<grid_p, kBlock, 0, h->stream>>>(aos_dev, pair32(h));
   else
-    aos_to_soa32<<<nblocks(h->g.vh), kBlock, 0, h->stream>>>(aos_dev, links32(h), h->g.vh);
+    aos_to_soa<<<grid, kBlock, 0, h->stream>>>(aos_dev, links32(h), h->g.vh);
   LAUNCH_CHECK(h);
   return QCD_OK;
 }
 
 int qcd_store_config_device(qcd_lattice* h, double* aos_dev) {
   if (!h || !aos_dev) return QCD_ERR_INVALID;
+  const dim3 grid(nblocks(h->g.vh), 2), grid_p((unsigned int)((h->gh.vh + kAosPairs - 1) / kAosPairs), 2);
   if (h->p.precision == QCD_PREC_FP64)
-    soa_to_aos64<<<nblocks(h->g.vh), kBlock, 0, h->stream>>>(links64(h), aos_dev, h->g.vh);
+    soa_to_aos<<<grid, kBlock, 0, h->stream>>>(links64(h), aos_dev, h->g.vh);
   else if (h->paired)
-    pair32_to_aos<<<nblocks(h->g.vh), kBlock, 0, h->stream>>>(pair32(h), aos_dev, h->g.vh);
+    pair32_to_aos<<<grid_p, kBlock, 0, h->stream>>>(pair32(h), aos_dev);
   else
-    soa_to_aos32<<<nblocks(h->g.vh), kBlock, 0, h->stream>>>(links32(h), aos_dev, h->g.vh);
+    soa_to_aos<<<grid, kBlock, 0, h->stream>>>(links32(h), aos_dev, h->g.vh);
   LAUNCH_CHECK(h);
   return QCD_OK;
 }
