@@ -299,9 +299,21 @@ struct PhiloxStream {
     philox_block_rk(ctr, ks, o);
     ctr[1]++;
   }
-  // (k + 1) / 2^24 for the top 24 bits k of a word: exact floats in (0, 1]
-  __device__ __forceinline__ static float u24(uint32_t w) { return (float)((w >> 8) + 1u) * 5.9604644775390625e-8f; }
-  __device__ __forceinline__ float uniform() { return u24(next()); }
+  // block b of a site's stream
+  __device__ __forceinline__ static void block_at(const PhiloxKeys& keys, uint32_t site, uint32_t b,
+                                                  unsigned long long phase, uint32_t o[4]) {
+    const uint32_t ctr[4] = {site, b, (uint32_t)phase, (uint32_t)(phase >> 32)};
+    philox_block_rk(ctr, keys, o);
+  }
+  // a u + c for the draw u = (k + 1) / 2^24 in (0, 1] of the top 24 bits k of a
+  // word, in one multiply-add: exact (no rounding) for the (a, c) the updates
+  // use, (1, 0), (1, -1/2), (2, -1) and (-1, 1), whose values are multiples of
+  // a / 2^24 that 24 bits hold
+  static constexpr float kU24 = 5.9604644775390625e-8f;
+  __device__ __forceinline__ static float u24(uint32_t w, float a = 1.f, float c = 0.f) {
+    return __fmaf_rn((float)(w >> 8), a * kU24, a * kU24 + c);
+  }
+  __device__ __forceinline__ float uniform(float a = 1.f, float c = 0.f) { return u24(next(), a, c); }
   // (k + 1) / 2^53 from 53 bits of two words: exact doubles in (0, 1]
   __device__ __forceinline__ double uniform_double() {
     const uint64_t hi = next(), lo = next();

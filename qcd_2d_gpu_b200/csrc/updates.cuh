@@ -15,6 +15,7 @@
 #pragma once
 #include <curand_kernel.h>
 #include "lattice.cuh"
+#include "rng.cuh"
 #include "su2.cuh"
 
 namespace qcd {
@@ -187,6 +188,54 @@ __device__ __forceinline__ Quat<double> overrelax_ref(Quat<double> A, const Quat
 // try of the rejection loop takes one block (r0, r1, r2 and the accept
 // uniform), the direction the first two words of the next one, the same
 // words in the same order as drawing them one by one.
+//
+// The phase is bound by instruction issue, so the steps are written out short:
+// exact one-step forms of the draws (PhiloxStream::u24), hardware log, sin and
+// cos without the handling of denormals their arguments never are (the
+// results are __logf's, __cosf's and __sincosf's on all 2^24 draws), and the
+// accept test in double only where single precision cannot decide it.
+__device__ __forceinline__ float log2_normal(float x) {  // __logf(x) = ln 2 log2_normal(x)
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float cos_normal(float x) {
+  float y;
+  asm("cos.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sin_normal(float x) {
+  float y;
+  asm("sin.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// one block of a try: t = log r0 + cos^2(2 pi r1) log r2 and 1 - the accept uniform
+// (hardware approximations, absolute error ~2^-21: the cosine is taken of
+// 2 pi (r1 - 1/2), which keeps the argument in [-pi, pi] and only flips the sign)
+__device__ __forceinline__ void heatbath_try(const uint32_t w[4], float& t, float& aux) {
+  const float c = cos_normal(6.2831853f * PhiloxStream::u24(w[1], 1.f, -0.5f));
+  const float ln2 = 0.693147182464599609375f;
+  t = __fmaf_rn(log2_normal(PhiloxStream::u24(w[0])), ln2,
+                __fmul_rn(__fmul_rn(c, c), __fmul_rn(log2_normal(PhiloxStream::u24(w[2])), ln2)));
+  aux = PhiloxStream::u24(w[3], -1.f, 1.f);
+}
+// aux^2 > 1 - lf in double.  The single-precision estimate of aux^2 + lf - 1 is
+// off by less than 4e-7 for lf < 2, and above it the sign is plain; a NaN
+// goes to the test in double.
+__device__ __forceinline__ bool heatbath_reject(float aux, float lf) {
+  const float v = __fmaf_rn(aux, aux, lf - 1.f);
+  if (fabsf(v) > 1e-6f) return v > 0.f;
+  return (double)aux * aux > 1.0 - (double)lf;
+}
+// direction of the spatial part from the first two words of a block
+__device__ __forceinline__ void heatbath_direction(const uint32_t w[4], float& ct, float& stt, float& cp, float& sp) {
+  ct = PhiloxStream::u24(w[0], 2.f, -1.f);
+  const float angle = 6.2831853f * PhiloxStream::u24(w[1], 1.f, -0.5f);  // angle + pi
+  sp = sin_normal(angle);
+  cp = cos_normal(angle);
+  stt = sqrtf(fmaxf(0.f, __fmaf_rn(-ct, ct, 1.f)));
+}
+
 template <class G>
 __device__ __forceinline__ Quat<float> heatbath_fast(Quat<float> A, float beta, G& st, int* err) {
   float det = q_det(A);
@@ -194,17 +243,13 @@ __device__ __forceinline__ Quat<float> heatbath_fast(Quat<float> A, float beta, 
   float a = det * rinv;
   A = Quat<float>{A.w * rinv, A.x * rinv, A.y * rinv, A.z * rinv};
   float inv = 0.5f / (a * beta);
-  float lf;
+  float lf, t, aux;
   uint32_t w[4];
   for (int tries = 1;; tries++) {
     st.block(w);
-    const float r0 = G::u24(w[0]), r1 = G::u24(w[1]), r2 = G::u24(w[2]);
-    // hardware approximations (absolute error ~2^-21): cos(2 pi r1) evaluated
-    // as -cos(2 pi (r1 - 1/2)) keeps the argument in [-pi, pi]
-    float c = -__cosf(6.2831853f * (r1 - 0.5f));
-    lf = -(__logf(r0) + c * c * __logf(r2)) * inv;
-    const float aux = 1.f - G::u24(w[3]);
-    if (!((double)aux * aux > 1.0 - (double)lf)) break;
+    heatbath_try(w, t, aux);
+    lf = -t * inv;
+    if (!heatbath_reject(aux, lf)) break;
     if (tries >= QCD_HB_MAX_TRIES) {
       atomicOr(err, DEVERR_HB_LOOP);
       break;
@@ -212,10 +257,9 @@ __device__ __forceinline__ Quat<float> heatbath_fast(Quat<float> A, float beta, 
   }
   const float x0 = 1.f - 2.f * lf;
   const float nrm = 2.f * sqrtf(lf * (1.f - lf));
+  float ct, stt, cp, sp;
   st.block(w);
-  float ct = 2.f * G::u24(w[0]) - 1.f, sp, cp;
-  __sincosf(6.2831853f * (G::u24(w[1]) - 0.5f), &sp, &cp);  // angle + pi
-  float stt = sqrtf(fmaxf(0.f, 1.f - ct * ct));
+  heatbath_direction(w, ct, stt, cp, sp);
   Quat<float> X{x0, nrm * ct, -nrm * stt * cp, -nrm * stt * sp};
   return q_mul_bd(X, A);
 }
@@ -239,9 +283,9 @@ __device__ __forceinline__ int metropolis_fast(Quat<float>& U, const Quat<float>
   int acc = 0;
   const float r0 = sqrtf(1.f - eps * eps);
   for (int h = 0; h < upd; h++) {
-    float r1 = st.uniform() - 0.5f;
-    float r2 = st.uniform() - 0.5f;
-    float r3 = st.uniform() - 0.5f;
+    float r1 = st.uniform(1.f, -0.5f);
+    float r2 = st.uniform(1.f, -0.5f);
+    float r3 = st.uniform(1.f, -0.5f);
     float sc = eps * rsqrtf(r1 * r1 + r2 * r2 + r3 * r3);
     Quat<float> r{r0, sc * r1, sc * r2, sc * r3};
     Quat<float> Un = q_mul(r, U);
@@ -256,12 +300,15 @@ __device__ __forceinline__ int metropolis_fast(Quat<float>& U, const Quat<float>
   return acc;
 }
 
-// Re-projection of an FP32 link with the norm taken in double.
+// Re-projection of an FP32 link with the norm taken in double.  An updated link
+// is within a few 1e-6 of the group, where 1/sqrt(1 + e) = 1 - e/2 + 3 e^2/8 has
+// an error of 5 e^3/16 < 4e-16, as good as rsqrt's in a third of the instructions.
 __device__ __forceinline__ Quat<float> renorm_fast(const Quat<float>& u) {
-  double d = (double)u.w * u.w + (double)u.x * u.x + (double)u.y * u.y + (double)u.z * u.z;
-  double inv = rsqrt(d);
-  return Quat<float>{(float)(u.w * inv), (float)(u.x * inv), (float)(u.y * inv),
-                     (float)(u.z * inv)};
+  const double w = u.w, x = u.x, y = u.y, z = u.z;
+  const double e = __fma_rn(w, w, __fma_rn(x, x, __fma_rn(y, y, __fma_rn(z, z, -1.0))));
+  double inv = __fma_rn(e, __fma_rn(e, 0.375, -0.5), 1.0);
+  if (!(fabs(e) < 1e-5)) inv = rsqrt(w * w + x * x + y * y + z * z);
+  return Quat<float>{(float)(w * inv), (float)(x * inv), (float)(y * inv), (float)(z * inv)};
 }
 
 }  // namespace qcd
