@@ -13,7 +13,7 @@
 // only difference is at the row seam: going +t from row Lt/2 - 1 (or -t from
 // row 0) lands on row 0 (Lt/2 - 1) with the two lanes exchanged, so the
 // loaded pair is swapped there.  The seam is a whole row, so the swap is
-// uniform over a CTA (a CTA works on one row).
+// uniform over a warp (a warp works on one row).
 //
 // The per-link arithmetic is the FP32 path's (updates.cuh): staples in FP32,
 // the heat-bath with its FP64 accept test and the Metropolis exact decision
@@ -305,18 +305,15 @@ __device__ __forceinline__ Q2 pair_update(const PS& P, const Geo& gh, const Phas
   return U;
 }
 
-// Launch grid (ceil(slice / kBlock), Lt/2): blockIdx.y is the row.  The
-// heat-bath and over-relaxation phases run spill-free at four CTAs per SM (64
-// registers), measured 3-5% faster than five with small spills; Metropolis
-// keeps five.
+// Launch grid tile_grid(gh), kTileThreads threads (the rows of the half geometry
+// are its t-slices; Lt/2 is even).  Every kind runs spill-free at eight CTAs per
+// SM (64 registers), measured 3-5% faster than ten with small spills.
 template <int MU, int PAR, int BC, int KIND>
-__global__ void __launch_bounds__(kBlock, KIND == KIND_METRO ? 5 : 4) phase32p(Pair32 P, Geo gh, PhaseArgs a) {
-  const int s = blockIdx.x * kBlock + threadIdx.x;
-  if (s >= gh.slice) return;
-  const int r = blockIdx.y;
-  const Nbr n = make_nbr_slice(gh, s, r, PAR);
+__global__ void __launch_bounds__(kTileThreads, 8) phase32p(Pair32 P, Geo gh, PhaseArgs a) {
+  Nbr n;
+  if (!tile_nbr<PAR>(gh, n)) return;
   if (BC == BC_PCC && MU != DIR_Y && at_y0(gh, n)) return;
-  P.st(MU, PAR, n.id, pair_update<MU, PAR, BC, KIND>(P, gh, a, n, r == gh.lt - 1, r == 0, a.renorm));
+  P.st(MU, PAR, n.id, pair_update<MU, PAR, BC, KIND>(P, gh, a, n, n.t == gh.lt - 1, n.t == 0, a.renorm));
 }
 
 // ------------------------------------------------------- measurement ----

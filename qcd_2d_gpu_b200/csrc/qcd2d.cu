@@ -201,16 +201,15 @@ Phase32pFn phase_fn32p(int k, int bc, int kind) {
 // only) every link is re-projected as it is stored
 int pass(qcd_lattice* h, int kind, int renorm = 0) {
   PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, renorm, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
-  const dim3 grid(nblocks(h->g.slice), (unsigned int)h->g.lt);
-  const dim3 grid_p(nblocks(h->gh.slice), (unsigned int)h->gh.lt);
+  const dim3 grid = tile_grid(h->g), grid_p = tile_grid(h->gh);
   for (int k = 0; k < 6; k++) {
     a.phase_off = (unsigned int)k;
     if (h->paired)
-      phase_fn32p(k, h->p.boundary, kind)<<<grid_p, kBlock, 0, h->stream>>>(pair32(h), h->gh, a);
+      phase_fn32p(k, h->p.boundary, kind)<<<grid_p, kTileThreads, 0, h->stream>>>(pair32(h), h->gh, a);
     else if (h->p.precision == QCD_PREC_FP64)
-      phase_fn64(k, h->p.boundary, kind)<<<grid, kBlock, 0, h->stream>>>(links64(h), rngs(h), h->g, a);
+      phase_fn64(k, h->p.boundary, kind)<<<grid, kTileThreads, 0, h->stream>>>(links64(h), rngs(h), h->g, a);
     else
-      phase_fn32(k, h->p.boundary, kind)<<<grid, kBlock, 0, h->stream>>>(links32(h), rngs(h), h->g, a);
+      phase_fn32(k, h->p.boundary, kind)<<<grid, kTileThreads, 0, h->stream>>>(links32(h), rngs(h), h->g, a);
     LAUNCH_CHECK(h);
   }
   if (kind != KIND_METRO) h->unit_passes++;
