@@ -845,13 +845,12 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
   if (serb) cudaMemcpyAsync(b->series, sv.ser, serb, cudaMemcpyDeviceToDevice, b->stream);
   cudaStreamSynchronize(b->stream);
   b->sweeps_done = swept;
-  if (rc) {
-    form_groups(b, bytes_save);
-    b->lanes = lanes_save;
-    return rc;
-  }
-  form_groups(b, best);
-  b->lanes = best_lanes;
+  // the kept grouping may have more groups than the saved counters and cursors
+  // were written for: give every group those of the first
+  form_groups(b, rc ? bytes_save : best);
+  spread_group_state<<<(b->n + 255) / 256, 256, 0, b->stream>>>(b->draw_dev, b->cursor, b->all_count, b->n);
+  b->lanes = rc ? lanes_save : best_lanes;
+  if (rc) return rc;
   if (bytes_out) *bytes_out = best;
   if (lanes_out) *lanes_out = best_lanes;
   if (ms_out) *ms_out = best_ms / sweeps_per_trial;
