@@ -300,15 +300,14 @@ __device__ __forceinline__ int metropolis_fast(Quat<float>& U, const Quat<float>
   return acc;
 }
 
-// Re-projection of an FP32 link with the norm taken in double.  An updated link
-// is within a few 1e-6 of the group, where 1/sqrt(1 + e) = 1 - e/2 + 3 e^2/8 has
-// an error of 5 e^3/16 < 4e-16, as good as rsqrt's in a third of the instructions.
+// Re-projection of an FP32 link with the norm taken in double.  (A series for
+// 1/sqrt near 1 saves about 20 instructions, but rounds one component in 10^9 to
+// the other neighbouring float, and a long chain does not forget that.)
 __device__ __forceinline__ Quat<float> renorm_fast(const Quat<float>& u) {
-  const double w = u.w, x = u.x, y = u.y, z = u.z;
-  const double e = __fma_rn(w, w, __fma_rn(x, x, __fma_rn(y, y, __fma_rn(z, z, -1.0))));
-  double inv = __fma_rn(e, __fma_rn(e, 0.375, -0.5), 1.0);
-  if (!(fabs(e) < 1e-5)) inv = rsqrt(w * w + x * x + y * y + z * z);
-  return Quat<float>{(float)(w * inv), (float)(x * inv), (float)(y * inv), (float)(z * inv)};
+  double d = (double)u.w * u.w + (double)u.x * u.x + (double)u.y * u.y + (double)u.z * u.z;
+  double inv = rsqrt(d);
+  return Quat<float>{(float)(u.w * inv), (float)(u.x * inv), (float)(u.y * inv),
+                     (float)(u.z * inv)};
 }
 
 }  // namespace qcd

@@ -29,7 +29,6 @@ def test_rejections_of_either_lane_match_the_unpaired_loop(dims, beta):
 
 @pytest.mark.parametrize("lt", [4, 6])  # site pairs and planes
 def test_reprojection_at_every_distance(lt):
-    # the series (|det - 1| < 1e-5) and the reciprocal square root meet at 1e-5
     rng = np.random.default_rng(8)
     n = lt * 4 * 8 * 3
     u = rng.normal(size=(n, 4))
