@@ -65,8 +65,11 @@ struct BatchArgs {
   int* err;
   int* accept;
   int renorm;
-  const unsigned long long* phase_ptr;  // drawing phases run so far (device word)
-  unsigned int phase_off;               // this phase's offset from it
+  // the drawing-phase counter of the launch (count_slots)
+  const unsigned long long* phase_ptr;
+  int phase_off;
+  unsigned long long* count_out;
+  unsigned int count_add;
 };
 
 template <int MU, int PAR, int KIND, bool FP64>
@@ -76,11 +79,14 @@ __global__ void __launch_bounds__(kBlock, 6) batch_phase(BatchView B, BatchArgs 
   const Replica& R = B.rep[r];
   const int id = (cta - R.cta_begin) * kBlock + threadIdx.x;
   if (id >= R.g.vh) return;
-  const Nbr n = make_nbr_fast(R.g, id, PAR);
+  Nbr n = make_nbr_fast(R.g, id, PAR);
+  chain_wait(n.id);
   // FP32 draws: the replica's seed as key, its stream offset added to the
   // site index, the batch-wide drawing-phase counter (as for one lattice)
   PhaseArgs pa{R.beta, a.eps, a.upd, a.err, a.accept ? a.accept + R.site_off : nullptr, a.renorm,
-               R.seed, a.phase_ptr, a.phase_off, (unsigned int)R.stream_off, philox_keys(R.seed)};
+               R.seed, a.phase_ptr, a.phase_off, (unsigned int)R.stream_off, philox_keys(R.seed), a.count_out,
+               a.count_add};
+  if (KIND != KIND_OR) count_draws(pa);
   RngStore RS{B.rng + R.rng_off, R.g.vh};
   if (FP64) {
     Links64 L{B.lo + R.link_off, B.hi + R.link_off, R.g.vh};
@@ -174,7 +180,6 @@ __global__ void __launch_bounds__(kBlock, FP64 ? kMeasurePerSM64 : kMeasurePerSM
   const int r = __ldg(B.mcta_rep + mcta);
   const Replica& R = B.rep[r];
   const int nblk = (int)measure_blocks(R.g.vh, FP64 ? kMeasurePerSM64 : kMeasurePerSM32);
-  const int k = *(volatile int*)cursor;  // advanced only by the last CTA below
   double e = 0, pl = 0;
   if (FP64) {
     Links64 L{B.lo + R.link_off, B.hi + R.link_off, R.g.vh};
@@ -189,6 +194,7 @@ __global__ void __launch_bounds__(kBlock, FP64 ? kMeasurePerSM64 : kMeasurePerSM
     else
       measure_sites<Links32, false>(L, R.g, mcta - R.mcta_begin, nblk, e, pl);
   }
+  const int k = *(volatile int*)cursor;  // advanced only by the last CTA below
   double se, sp;
   block_sum2(e, pl * (1.0 / 3.0), &se, &sp);
   __shared__ bool last_rep;
@@ -282,7 +288,8 @@ struct qcd_batch {
   uint32_t* rng = nullptr;
   uint32_t* mrg_jumps = nullptr;  // jump matrices that seed the streams (mrg_jump_table)
   // per group (n entries, groups use the first ones): drawing phases run so
-  // far (FP32 draws), arrival counter and cursor of the measurement
+  // far (FP32 draws; n more entries take it through a pass, count_slots),
+  // arrival counter and cursor of the measurement
   unsigned long long* draw_dev = nullptr;
   unsigned int* all_count = nullptr;
   int* cursor = nullptr;
@@ -387,18 +394,11 @@ __global__ void spread_group_state(unsigned long long* draw, int* cursor, unsign
 
 int batch_pass(qcd_batch* b, int gi, int kind, int renorm) {
   const BatchGroup& g = b->groups[gi];
-  BatchArgs a{b->common.epsilon, b->common.upd, b->err, b->accept, renorm, b->draw_dev + gi, 0};
+  BatchArgs a{b->common.epsilon, b->common.upd, b->err, b->accept, renorm};
   for (int k = 0; k < 6; k++) {
-    a.phase_off = (unsigned int)k;
-    if (fp64(b))
-      batch_phase_fn<true>(k, kind)<<<g.ctas, kBlock, 0, b->stream>>>(view(b, g), a);
-    else
-      batch_phase_fn<false>(k, kind)<<<g.ctas, kBlock, 0, b->stream>>>(view(b, g), a);
-    BCUDA(b, cudaGetLastError());
-  }
-  if (kind != KIND_OR) {
-    advance_counter<<<1, 1, 0, b->stream>>>(b->draw_dev + gi, 6ull);
-    BCUDA(b, cudaGetLastError());
+    count_slots(a, b->draw_dev + gi, b->draw_dev + b->n + gi, k, kind != KIND_OR);
+    BCUDA(b, launch_chained(fp64(b) ? batch_phase_fn<true>(k, kind) : batch_phase_fn<false>(k, kind), g.ctas, kBlock,
+                            b->stream, view(b, g), a));
   }
   return QCD_OK;
 }
@@ -424,13 +424,8 @@ int batch_sweep(qcd_batch* b, int gi, bool renorm) {
 
 int batch_measure_launch(qcd_batch* b, int gi) {
   const BatchGroup& g = b->groups[gi];
-  if (fp64(b))
-    batch_measure<true><<<g.mctas, kBlock, 0, b->stream>>>(view(b, g), b->partials, b->rep_count, b->all_count + gi,
-                                                           b->cursor + gi, b->series, b->cap);
-  else
-    batch_measure<false><<<g.mctas, kBlock, 0, b->stream>>>(view(b, g), b->partials, b->rep_count,
-                                                            b->all_count + gi, b->cursor + gi, b->series, b->cap);
-  BCUDA(b, cudaGetLastError());
+  BCUDA(b, launch_chained(fp64(b) ? batch_measure<true> : batch_measure<false>, g.mctas, kBlock, b->stream, view(b, g),
+                          b->partials, b->rep_count, b->all_count + gi, b->cursor + gi, b->series, b->cap));
   return QCD_OK;
 }
 
@@ -569,7 +564,7 @@ int qcd_batch_create(const qcd_replica* r, int n, const qcd_params* common, qcd_
     if (rc == QCD_OK) step(cudaMemsetAsync(b->accept, 0, site_off * sizeof(int), b->stream), "memset");
   }
   if (rc == QCD_OK) step(cudaMalloc(&b->err, sizeof(int)), "cudaMalloc(err)");
-  if (rc == QCD_OK) step(cudaMalloc(&b->draw_dev, n * sizeof(unsigned long long)), "cudaMalloc(draw counters)");
+  if (rc == QCD_OK) step(cudaMalloc(&b->draw_dev, 2 * n * sizeof(unsigned long long)), "cudaMalloc(draw counters)");
   if (rc == QCD_OK) step(cudaMemsetAsync(b->draw_dev, 0, n * sizeof(unsigned long long), b->stream), "memset");
   if (rc == QCD_OK)
     step(cudaMalloc(&b->partials, (size_t)(mcta > cta ? mcta : cta) * sizeof(double2)), "cudaMalloc(partials)");

@@ -19,13 +19,17 @@ namespace qcd {
 template <int MU, int PAR, int BC, int KIND>
 __global__ void __launch_bounds__(kTileThreads, KIND == KIND_OR ? 8 : KIND == KIND_HB ? 9 : 6) phase64(Links64 L, RngStore R, Geo g, PhaseArgs a) {
   Nbr n;
-  if (tile_nbr<PAR>(g, n)) site64<MU, PAR, BC, KIND, false>(L, R, g, a, n);
+  if (!tile_nbr<PAR>(g, n)) return;
+  if (KIND != KIND_OR) count_draws(a);
+  site64<MU, PAR, BC, KIND, false>(L, R, g, a, n);
 }
 
 template <int MU, int PAR, int BC, int KIND>
 __global__ void __launch_bounds__(kTileThreads) phase32(Links32 L, RngStore R, Geo g, PhaseArgs a) {
   Nbr n;
-  if (tile_nbr<PAR>(g, n)) site32<MU, PAR, BC, KIND, false>(L, R, g, a, n, a.renorm);
+  if (!tile_nbr<PAR>(g, n)) return;
+  if (KIND != KIND_OR) count_draws(a);
+  site32<MU, PAR, BC, KIND, false>(L, R, g, a, n, a.renorm);
 }
 
 // ------------------------------------------------------------ RNG setup --

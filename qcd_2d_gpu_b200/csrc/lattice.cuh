@@ -132,7 +132,37 @@ __host__ __forceinline__ dim3 tile_grid(const Geo& g) {  // Lt and Lx are even
   return dim3((unsigned int)((g.lyh * (g.lx / 2) + kTileY - 1) / kTileY), (unsigned int)(g.lt / 2));
 }
 
-// The site of this thread; false beyond the end of the slice pair.
+// Launches follow one another by programmatic dependence (launch_chained): the
+// CTAs of a launch are set up while its predecessor drains, and wait here until
+// the predecessor has completed and its writes are visible.  A kernel launched
+// so reads and writes global memory only after chain_wait, through a value that
+// went through it (an asm operand, so that no load can be moved above), and
+// calls chain_ready when its CTA has little left to do.  Calling chain_ready
+// just before the store is best over all sizes; as the first thing, the CTAs of
+// launches to come take up slots (54x62x70 heat-bath pass 35.7 us against 29.8),
+// never, the set-up is exposed again at the large sizes.  Passes without and
+// with the chain: 16^3 FP64 40 -> 25 us, 24x20x28 28 -> 17, 54x62x70 39 -> 30,
+// 128^3 FP32 over-relaxation 103 -> 90, heat-bath 149 -> 133.
+__device__ __forceinline__ void chain_wait(unsigned int& x) { asm volatile("griddepcontrol.wait;" : "+r"(x)::"memory"); }
+__device__ __forceinline__ void chain_wait(int& x) { asm volatile("griddepcontrol.wait;" : "+r"(x)::"memory"); }
+__device__ __forceinline__ void chain_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+__host__ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int block, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned int)block);
+  c.stream = stream;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+// The site of this thread, after the wait for the preceding launch; false
+// beyond the end of the slice pair.
 template <int PAR>
 __device__ __forceinline__ bool tile_nbr(const Geo& g, Nbr& n) {
   const int u = blockIdx.x * kTileY + threadIdx.x % kTileY, w = threadIdx.x / kTileY;
@@ -143,6 +173,7 @@ __device__ __forceinline__ bool tile_nbr(const Geo& g, Nbr& n) {
   n.yq = u - xp * g.lyh;
   n.id = n.yq + g.lyh * n.x + g.slice * n.t;
   finish_nbr(g, PAR, n);
+  chain_wait(n.id);
   return true;
 }
 
@@ -165,16 +196,14 @@ __host__ __device__ __forceinline__ size_t plane_of(int dir, int parity) { retur
 // links, which is safe inside one phase launch because no link a phase reads
 // is written in that launch.  CG = true (the wavefront kernel) reads and
 // writes at L2 (.cg): there, other CTAs of the same launch rewrite links, and
-// a line left in this SM's L1 by an earlier task could be stale.
+// a line left in this SM's L1 by an earlier task could be stale.  The link a
+// thread rewrites is read at L2 in either case: its sector may hold a link that
+// another SM rewrites in the same launch, and the next launch's CTAs may already
+// be set up on this SM.
 template <class T, bool CG>
 __device__ __forceinline__ T ld_nb(const T* p) {
   if (CG) return __ldcg(p);
   return __ldg(p);
-}
-template <class T, bool CG>
-__device__ __forceinline__ T ld_rw(const T* p) {
-  if (CG) return __ldcg(p);
-  return *p;
 }
 template <class T, bool CG>
 __device__ __forceinline__ void st_rw(T* p, const T& v) {
@@ -198,7 +227,7 @@ struct Links64T {
   // the link this thread rewrites
   __device__ __forceinline__ Quat<double> ld_own(int dir, int parity, int id) const {
     size_t i = plane_of(dir, parity) * vh + id;
-    double2 a = ld_rw<double2, CG>(lo + i), b = ld_rw<double2, CG>(hi + i);
+    double2 a = __ldcg(lo + i), b = __ldcg(hi + i);
     return Quat<double>{a.x, a.y, b.x, b.y};
   }
   __device__ __forceinline__ void st(int dir, int parity, int id, const Quat<double>& u) const {
@@ -219,7 +248,7 @@ struct Links32T {
     return Quat<float>{a.x, a.y, a.z, a.w};
   }
   __device__ __forceinline__ Quat<float> ld_own(int dir, int parity, int id) const {
-    float4 a = ld_rw<float4, CG>(q + plane_of(dir, parity) * vh + id);
+    float4 a = __ldcg(q + plane_of(dir, parity) * vh + id);
     return Quat<float>{a.x, a.y, a.z, a.w};
   }
   __device__ __forceinline__ void st(int dir, int parity, int id, const Quat<float>& u) const {

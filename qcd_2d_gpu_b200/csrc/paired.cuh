@@ -104,7 +104,7 @@ __device__ __forceinline__ Q2 ld_pair_nc(const float4* p) {
 }
 __device__ __forceinline__ Q2 ld_pair(const float4* p) {
   float a0, a1, a2, a3, b0, b1, b2, b3;
-  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+  asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=f"(a0), "=f"(a1), "=f"(a2), "=f"(a3), "=f"(b0), "=f"(b1), "=f"(b2), "=f"(b3)
                : "l"(p)
                : "memory");
@@ -295,8 +295,8 @@ __device__ __forceinline__ Q2 pair_update(const PS& P, const Geo& gh, const Phas
     const int acc0 = metropolis_fast(u0, lane0(A), a.beta, a.eps, a.upd, s0);
     const int acc1 = metropolis_fast(u1, lane1(A), a.beta, a.eps, a.upd, s1);
     int* acc = a.accept + PAR * 2 * P.vhp;
-    acc[gid0] += acc0;
-    acc[gid1] += acc1;
+    atomicAdd(acc + gid0, acc0);
+    atomicAdd(acc + gid1, acc1);
     U = join(u0, u1);
   } else {
     U = overrelax2(A, P.ld_own(MU, PAR, n.id));
@@ -312,8 +312,11 @@ template <int MU, int PAR, int BC, int KIND>
 __global__ void __launch_bounds__(kTileThreads, 8) phase32p(Pair32 P, Geo gh, PhaseArgs a) {
   Nbr n;
   if (!tile_nbr<PAR>(gh, n)) return;
+  if (KIND != KIND_OR) count_draws(a);
   if (BC == BC_PCC && MU != DIR_Y && at_y0(gh, n)) return;
-  P.st(MU, PAR, n.id, pair_update<MU, PAR, BC, KIND>(P, gh, a, n, n.t == gh.lt - 1, n.t == 0, a.renorm));
+  const Q2 U = pair_update<MU, PAR, BC, KIND>(P, gh, a, n, n.t == gh.lt - 1, n.t == 0, a.renorm);
+  chain_ready();
+  P.st(MU, PAR, n.id, U);
 }
 
 // ------------------------------------------------------- measurement ----
@@ -337,8 +340,8 @@ template <bool PMC>
 __device__ __forceinline__ void measure_pairs(const Pair32& P, const Geo& gh, int c, int nb, double& e, double& pl) {
   const int p = threadIdx.x >= kMeasureIds;
   const unsigned int pairs = (unsigned int)gh.vh;
-  for (unsigned int k = (unsigned int)c * kMeasureIds + threadIdx.x % kMeasureIds; k < pairs;
-       k += (unsigned int)nb * kMeasureIds) {
+  unsigned int k = (unsigned int)c * kMeasureIds + threadIdx.x % kMeasureIds;
+  for (chain_wait(k); k < pairs; k += (unsigned int)nb * kMeasureIds) {
     const int id = (int)k;
     const int r = div_by(k, gh.slice_m);
     const int s = id - r * gh.slice;
@@ -356,6 +359,7 @@ __device__ __forceinline__ void measure_pairs(const Pair32& P, const Geo& gh, in
     e += -cs;
     pl += 6 - ay - by - cs;
   }
+  chain_ready();
 }
 
 template <int PMC>

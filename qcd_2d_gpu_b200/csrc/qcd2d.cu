@@ -57,7 +57,7 @@ struct qcd_lattice {
   long long sweeps_done = 0;
   // drawing phases run so far (6 per heat-bath or Metropolis pass), on the
   // device: the counter of the FP32 Philox draws, part of the generator
-  // checkpoint
+  // checkpoint, and the word that takes it through a pass (count_slots)
   unsigned long long* draw_dev = nullptr;
   unsigned long long draw_key = 0;  // key of the FP32 draws: the seed, or the one a checkpoint restored
   // wavefront scheduler
@@ -203,20 +203,18 @@ int pass(qcd_lattice* h, int kind, int renorm = 0) {
   PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, renorm, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
   const dim3 grid = tile_grid(h->g), grid_p = tile_grid(h->gh);
   for (int k = 0; k < 6; k++) {
-    a.phase_off = (unsigned int)k;
+    count_slots(a, h->draw_dev, h->draw_dev + 1, k, kind != KIND_OR);
     if (h->paired)
-      phase_fn32p(k, h->p.boundary, kind)<<<grid_p, kTileThreads, 0, h->stream>>>(pair32(h), h->gh, a);
+      CUDA_OR_FAIL(h, launch_chained(phase_fn32p(k, h->p.boundary, kind), grid_p, kTileThreads, h->stream, pair32(h),
+                                     h->gh, a));
     else if (h->p.precision == QCD_PREC_FP64)
-      phase_fn64(k, h->p.boundary, kind)<<<grid, kTileThreads, 0, h->stream>>>(links64(h), rngs(h), h->g, a);
+      CUDA_OR_FAIL(h, launch_chained(phase_fn64(k, h->p.boundary, kind), grid, kTileThreads, h->stream, links64(h),
+                                     rngs(h), h->g, a));
     else
-      phase_fn32(k, h->p.boundary, kind)<<<grid, kTileThreads, 0, h->stream>>>(links32(h), rngs(h), h->g, a);
-    LAUNCH_CHECK(h);
+      CUDA_OR_FAIL(h, launch_chained(phase_fn32(k, h->p.boundary, kind), grid, kTileThreads, h->stream, links32(h),
+                                     rngs(h), h->g, a));
   }
   if (kind != KIND_METRO) h->unit_passes++;
-  if (kind != KIND_OR) {
-    advance_counter<<<1, 1, 0, h->stream>>>(h->draw_dev, 6ull);
-    LAUNCH_CHECK(h);
-  }
   return QCD_OK;
 }
 
@@ -447,7 +445,7 @@ int launch_wave(qcd_lattice* h, const PassSpec* ps, int np, int stall_test = 0,
   const int sk = h->p.algo == QCD_ALGO_HEATBATH ? KIND_HB : KIND_METRO;
   const int bc = h->p.boundary;
   const unsigned int grid = (unsigned int)h->wave_grid;
-  RngStoreT<true> R{h->rng, h->g.vh};
+  RngStore R{h->rng, h->g.vh};
   if (h->p.precision == QCD_PREC_FP64) {
     Links64T<true> L{h->lo, h->hi, h->g.vh};
     if (sk == KIND_HB) {
@@ -578,23 +576,28 @@ int launch_measure(qcd_lattice* h, double* out_dev, const int* err) {
   if (h->p.precision == QCD_PREC_FP64) {
     const unsigned int nb = measure_blocks(h->g.vh, kMeasurePerSM64);
     if (pmc)
-      measure<Links64, 1, kMeasurePerSM64><<<nb, kBlock, 0, h->stream>>>(links64(h), h->g, h->partials, h->counter, out_dev, err);
+      CUDA_OR_FAIL(h, launch_chained(measure<Links64, 1, kMeasurePerSM64>, nb, kBlock, h->stream, links64(h), h->g, h->partials,
+                                     h->counter, out_dev, err));
     else
-      measure<Links64, 0, kMeasurePerSM64><<<nb, kBlock, 0, h->stream>>>(links64(h), h->g, h->partials, h->counter, out_dev, err);
+      CUDA_OR_FAIL(h, launch_chained(measure<Links64, 0, kMeasurePerSM64>, nb, kBlock, h->stream, links64(h), h->g, h->partials,
+                                     h->counter, out_dev, err));
   } else if (h->paired) {
     const unsigned int nb = measure_blocks(h->gh.vh, kMeasurePerSMPair);
     if (pmc)
-      measure_p<1><<<nb, kBlock, 0, h->stream>>>(pair32(h), h->gh, h->partials, h->counter, out_dev, err);
+      CUDA_OR_FAIL(h, launch_chained(measure_p<1>, nb, kBlock, h->stream, pair32(h), h->gh, h->partials,
+                                     h->counter, out_dev, err));
     else
-      measure_p<0><<<nb, kBlock, 0, h->stream>>>(pair32(h), h->gh, h->partials, h->counter, out_dev, err);
+      CUDA_OR_FAIL(h, launch_chained(measure_p<0>, nb, kBlock, h->stream, pair32(h), h->gh, h->partials,
+                                     h->counter, out_dev, err));
   } else {
     const unsigned int nb = measure_blocks(h->g.vh, kMeasurePerSM32);
     if (pmc)
-      measure<Links32, 1, kMeasurePerSM32><<<nb, kBlock, 0, h->stream>>>(links32(h), h->g, h->partials, h->counter, out_dev, err);
+      CUDA_OR_FAIL(h, launch_chained(measure<Links32, 1, kMeasurePerSM32>, nb, kBlock, h->stream, links32(h), h->g, h->partials,
+                                     h->counter, out_dev, err));
     else
-      measure<Links32, 0, kMeasurePerSM32><<<nb, kBlock, 0, h->stream>>>(links32(h), h->g, h->partials, h->counter, out_dev, err);
+      CUDA_OR_FAIL(h, launch_chained(measure<Links32, 0, kMeasurePerSM32>, nb, kBlock, h->stream, links32(h), h->g, h->partials,
+                                     h->counter, out_dev, err));
   }
-  LAUNCH_CHECK(h);
   return QCD_OK;
 }
 
@@ -751,7 +754,7 @@ int qcd_create(const qcd_params* p, qcd_lattice** out) {
   if (rc == QCD_OK) step(cudaMalloc(&h->partials, nb * sizeof(double2)), "cudaMalloc(partials)");
   if (rc == QCD_OK) step(cudaMalloc(&h->counter, sizeof(unsigned int)), "cudaMalloc(counter)");
   if (rc == QCD_OK) step(cudaMalloc(&h->err, sizeof(int)), "cudaMalloc(err)");
-  if (rc == QCD_OK) step(cudaMalloc(&h->draw_dev, sizeof(unsigned long long)), "cudaMalloc(draw counter)");
+  if (rc == QCD_OK) step(cudaMalloc(&h->draw_dev, 2 * sizeof(unsigned long long)), "cudaMalloc(draw counter)");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->draw_dev, 0, sizeof(unsigned long long), h->stream), "memset");
   if (rc == QCD_OK) step(cudaMallocHost(&h->result_host, 4 * sizeof(double)), "cudaMallocHost");
   if (rc == QCD_OK) step(cudaHostGetDevicePointer((void**)&h->result_dev, h->result_host, 0), "cudaHostGetDevicePointer");

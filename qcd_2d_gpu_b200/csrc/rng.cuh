@@ -16,21 +16,17 @@
 
 namespace qcd {
 
-template <bool CG>
-struct RngStoreT {
+// Reads and writes go to L2: a word is rewritten by every drawing phase, perhaps
+// from another SM, while 32-B sectors hold the words of several CTAs' sites.
+struct RngStore {
   uint32_t* w;  // w[j * vh + id], j = 0..2 -> s1[j], j = 3..5 -> s2[j-3]
   int vh;
 
   __device__ __forceinline__ uint32_t get(int j, int id) const {
-    const uint32_t* p = w + (size_t)j * vh + id;
-    return CG ? __ldcg(p) : *p;
+    return __ldcg(w + (size_t)j * vh + id);
   }
   __device__ __forceinline__ void put(int j, int id, uint32_t v) const {
-    uint32_t* p = w + (size_t)j * vh + id;
-    if (CG)
-      __stcg(p, v);
-    else
-      *p = v;
+    __stcg(w + (size_t)j * vh + id, v);
   }
   __device__ __forceinline__ void load(int id, curandStateMRG32k3a_t* s) const {
     s->s1[0] = get(0, id);
@@ -53,7 +49,6 @@ struct RngStoreT {
     put(5, id, s->s2[2]);
   }
 };
-typedef RngStoreT<false> RngStore;
 
 // ------------------------------------------------- seeding many streams ----
 // curand_init(seed, id, 0) places stream id 2^76 steps after stream id - 1

@@ -20,44 +20,58 @@ struct PhaseArgs {
   int* err;     // device error word
   int* accept;  // V ints, reference site order; only for Metropolis
   int renorm;   // FP32: re-project each updated link (in double) before it is stored
-  // FP32 draws (counter-based): the key, the device word holding the number
-  // of drawing phases run before this launch (advanced on the device, so a
-  // captured graph draws fresh numbers on every replay), this phase's offset
-  // from it, and the offset added to the site index (a replica's stream
-  // offset in a batch)
+  // FP32 draws (counter-based): the key, a device word that counts drawing
+  // phases (advanced on the device, so a captured graph draws fresh numbers on
+  // every replay), this phase's offset from it, and the offset added to the
+  // site index (a replica's stream offset in a batch)
   unsigned long long seed;
   const unsigned long long* phase_ptr;
-  unsigned int phase_off;
+  int phase_off;
   unsigned int site_off;
   PhiloxKeys keys;  // round keys of `seed` (philox_keys), set by whoever fills the arguments
+  // where this launch writes the count for later launches (count_draws), or null
+  unsigned long long* count_out = nullptr;
+  unsigned int count_add = 0;
 };
 
-// The drawing-phase counter of the FP32 draws lives on the device and is
-// advanced by this one-thread launch after every heat-bath or Metropolis pass
-// (inside a captured graph too).  Internal linkage: each translation unit
-// that includes this header has its own copy.
-static __global__ void advance_counter(unsigned long long* c, unsigned long long n) { *c += n; }
-
+// The drawing-phase counter lives on the device as two words, both holding the
+// count between passes; the first is the one that is saved and restored.  A
+// drawing pass advances it without a launch of its own (2 us each before): phases
+// 0-2 read word 0 while phase 0 writes the advanced count to word 1, phases 3-5
+// read word 1 while phase 3 copies it back, so no launch writes the word it reads.
+template <class Args>
+__host__ inline void count_slots(Args& a, unsigned long long* word0, unsigned long long* word1, int k, bool draws) {
+  a.phase_ptr = k < 3 ? word0 : word1;
+  a.phase_off = k < 3 ? k : k - 6;
+  a.count_out = !draws ? nullptr : k == 0 ? word1 : k == 3 ? word0 : nullptr;
+  a.count_add = k == 0 ? 6 : 0;
+}
+__device__ __forceinline__ unsigned long long draw_count(const PhaseArgs& a) {
+  const unsigned long long* p = a.phase_ptr;
+  asm volatile("" : "+l"(p));  // after chain_wait
+  return __ldg(p);
+}
+__device__ __forceinline__ void count_draws(const PhaseArgs& a) {
+  if (a.count_out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+    __stcg(a.count_out, draw_count(a) + a.count_add);
+}
 // the drawing-phase number of this launch
 __device__ __forceinline__ unsigned long long draw_phase(const PhaseArgs& a) {
-  return __ldg(a.phase_ptr) + a.phase_off;
+  return draw_count(a) + (long long)a.phase_off;
 }
+
+// The wavefront and the fused pairs, which read word 0 alone, advance it by this
+// one-thread launch (inside a captured graph too).  Internal linkage: each
+// translation unit that includes this header has its own copy.
+static __global__ void advance_counter(unsigned long long* c, unsigned long long n) { *c += n; }
 
 // ------------------------------------------------------- one link update --
 // Update U_MU at site n of sublattice PAR: the body of the six launches of
 // mc_up_per/pcc/pmc (mc_updates.h:129-465, mc_updates_pcc.h:4-214,
 // mc_updates_pmc.h:4-247).  Shared by the per-phase kernels (CG = false) and
 // the wavefront kernel (CG = true).
-template <bool CG>
-__device__ __forceinline__ void add_accept(int* p, int v) {
-  if (CG)
-    atomicAdd(p, v);  // at L2: the counter may sit in a stale L1 line
-  else
-    *p += v;
-}
-
 template <int MU, int PAR, int BC, int KIND, bool CG>
-__device__ __forceinline__ void site64(const Links64T<CG>& L, const RngStoreT<CG>& R, const Geo& g,
+__device__ __forceinline__ void site64(const Links64T<CG>& L, const RngStore& R, const Geo& g,
                                        const PhaseArgs& a, const Nbr& n) {
   if (BC == BC_PCC && MU != DIR_Y && at_y0(g, n)) return;
   const int id = n.id;
@@ -66,6 +80,7 @@ __device__ __forceinline__ void site64(const Links64T<CG>& L, const RngStoreT<CG
     curandStateMRG32k3a_t st;
     R.load(id, &st);
     Quat<double> U = heatbath_ref(A, (double)a.beta, &st, a.err);
+    if (!CG) chain_ready();
     L.st(MU, PAR, id, U);
     R.store(id, &st);
   } else if (KIND == KIND_METRO) {
@@ -73,12 +88,14 @@ __device__ __forceinline__ void site64(const Links64T<CG>& L, const RngStoreT<CG
     R.load(id, &st);
     Quat<double> U = L.ld_own(MU, PAR, id);
     int acc = metropolis_ref(U, A, (double)a.beta, (double)a.eps, a.upd, &st);
+    if (!CG) chain_ready();
     L.st(MU, PAR, id, U);
     R.store(id, &st);
-    add_accept<CG>(a.accept + PAR * g.vh + id, acc);
+    atomicAdd(a.accept + PAR * g.vh + id, acc);
   } else {
-    Quat<double> U = L.ld_own(MU, PAR, id);
-    L.st(MU, PAR, id, overrelax_ref(A, U));
+    Quat<double> U = overrelax_ref(A, L.ld_own(MU, PAR, id));
+    if (!CG) chain_ready();
+    L.st(MU, PAR, id, U);
   }
 }
 
@@ -110,7 +127,7 @@ __device__ __forceinline__ Quat<float> link_update32(const L& links, const Geo& 
 }
 
 template <int MU, int PAR, int BC, int KIND, bool CG>
-__device__ __forceinline__ void site32(const Links32T<CG>& L, const RngStoreT<CG>& R, const Geo& g,
+__device__ __forceinline__ void site32(const Links32T<CG>& L, const RngStore& R, const Geo& g,
                                        const PhaseArgs& a, const Nbr& n, int renorm) {
   if (BC == BC_PCC && MU != DIR_Y && at_y0(g, n)) return;
   const int id = n.id;
@@ -123,11 +140,13 @@ __device__ __forceinline__ void site32(const Links32T<CG>& L, const RngStoreT<CG
     PhiloxStream st(a.keys, a.site_off + (unsigned int)id, draw_phase(a));
     U = L.ld_own(MU, PAR, id);
     int acc = metropolis_fast(U, A, a.beta, a.eps, a.upd, st);
-    add_accept<CG>(a.accept + PAR * g.vh + id, acc);
+    atomicAdd(a.accept + PAR * g.vh + id, acc);
   } else {
     U = overrelax_fast(A, L.ld_own(MU, PAR, id));
   }
-  L.st(MU, PAR, id, renorm ? renorm_fast(U) : U);
+  if (renorm) U = renorm_fast(U);
+  if (!CG) chain_ready();
+  L.st(MU, PAR, id, U);
 }
 
 // ---------------------------------------------------------- reductions --
@@ -264,8 +283,8 @@ template <class L, bool PMC>
 __device__ __forceinline__ void measure_sites(const L& links, const Geo& g, int c, int nb, double& e, double& pl) {
   const int p = threadIdx.x >= kMeasureIds;
   const unsigned int ids = (unsigned int)g.vh;
-  for (unsigned int k = (unsigned int)c * kMeasureIds + threadIdx.x % kMeasureIds; k < ids;
-       k += (unsigned int)nb * kMeasureIds) {
+  unsigned int k = (unsigned int)c * kMeasureIds + threadIdx.x % kMeasureIds;
+  for (chain_wait(k); k < ids; k += (unsigned int)nb * kMeasureIds) {
     const int id = (int)k;
     const int t = div_by(k, g.slice_m);
     const int s = id - t * g.slice;
@@ -280,6 +299,7 @@ __device__ __forceinline__ void measure_sites(const L& links, const Geo& g, int 
     e += -cc;
     pl += 3 - a - b - cc;  // the 1/3 of the plaquette average is applied once per thread
   }
+  chain_ready();
 }
 
 }  // namespace qcd

@@ -89,7 +89,7 @@ __device__ __forceinline__ long long wave_tasks_before(const WaveSched& S, int t
     break;
 
 template <int BC, int SK>
-__device__ __forceinline__ void wave_site(const Links64T<true>& L, const RngStoreT<true>& R, const Geo& g,
+__device__ __forceinline__ void wave_site(const Links64T<true>& L, const RngStore& R, const Geo& g,
                                           const PhaseArgs& a, int type, int kind, int rn, int s, int t) {
   switch (type) {
     QCD_WAVE_CASE64(DIR_Y, 0)
@@ -102,7 +102,7 @@ __device__ __forceinline__ void wave_site(const Links64T<true>& L, const RngStor
 }
 
 template <int BC, int SK>
-__device__ __forceinline__ void wave_site(const Links32T<true>& L, const RngStoreT<true>& R, const Geo& g,
+__device__ __forceinline__ void wave_site(const Links32T<true>& L, const RngStore& R, const Geo& g,
                                           const PhaseArgs& a, int type, int kind, int rn, int s, int t) {
   switch (type) {
     QCD_WAVE_CASE32(DIR_Y, 0)
@@ -117,7 +117,7 @@ __device__ __forceinline__ void wave_site(const Links32T<true>& L, const RngStor
 // LinksT: Links64T<true> or Links32T<true>; BC: boundary; SK: the sweep's
 // update kind (heat-bath or Metropolis); over-relaxation phases are KIND_OR.
 template <class LinksT, int BC, int SK>
-__global__ void __launch_bounds__(kBlock, 5) wave(LinksT L, RngStoreT<true> R, Geo g, PhaseArgs a,
+__global__ void __launch_bounds__(kBlock, 5) wave(LinksT L, RngStore R, Geo g, PhaseArgs a,
                                                   WaveSched S, WaveCtl c) {
   __shared__ int sh_ok, sh_n, sh_t, sh_chunk;
   // Thread 0 keeps one ticket in hand: the atomic for the next ticket is
