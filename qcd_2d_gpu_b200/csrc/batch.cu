@@ -119,18 +119,17 @@ __global__ void __launch_bounds__(kBlock) batch_setup(BatchView B, const uint32_
   __syncthreads();
   const int id = id0 + threadIdx.x;
   if (id >= R.g.vh) return;
-  curandStateMRG32k3a_t st;
-  mrg_jump_from(base, jumps, threadIdx.x, &st);
+  MrgStream st = mrg_jump_from(base, jumps, threadIdx.x);
   for (int p = 0; p < 2; p++) {
     const Nbr n = make_nbr(R.g, id, p);
     const bool frozen = R.bc == BC_PCC && at_y0(R.g, n);
     for (int d = 0; d < 3; d++) {
       Quat<double> u = q_one<double>();
       if (R.hot && !(d != DIR_Y && frozen)) {
-        u.w = curand_uniform_double(&st) - 0.5;
-        u.x = curand_uniform_double(&st) - 0.5;
-        u.y = curand_uniform_double(&st) - 0.5;
-        u.z = curand_uniform_double(&st) - 0.5;
+        u.w = st.uniform_double() - 0.5;
+        u.x = st.uniform_double() - 0.5;
+        u.y = st.uniform_double() - 0.5;
+        u.z = st.uniform_double() - 0.5;
         u = q_normalize(u);
       }
       if (FP64) {
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(kBlock) batch_setup(BatchView B, const uint32_
     }
   }
   RngStore RS{B.rng + R.rng_off, R.g.vh};
-  RS.store(id, &st);
+  RS.store(id, st);
 }
 
 template <bool FP64>

@@ -13,11 +13,12 @@
 namespace qcd {
 
 // ------------------------------------------------------------ one phase --
-// Launch grid tile_grid(g), kTileThreads threads.  FP64: eight CTAs per SM for
-// over-relaxation (64 registers; 128^3 phase 39.8 us at the compiler's choice,
-// 38.1 at eight, 40.3 at ten), nine for the heat-bath (54.5, 53.2 us).
+// Launch grid tile_grid(g), kTileThreads threads.  FP64 CTAs per SM, measured:
+// over-relaxation nine (56 registers; 128^3 pass 211 us, 216 at eight, 239 at the
+// compiler's choice), heat-bath and Metropolis seven (72; heat-bath 64^3 40.6 us,
+// 42.1 at nine, 45.8 at six; Metropolis 64^3 65.6 us, 72 at six).
 template <int MU, int PAR, int BC, int KIND>
-__global__ void __launch_bounds__(kTileThreads, KIND == KIND_OR ? 8 : KIND == KIND_HB ? 9 : 6) phase64(Links64 L, RngStore R, Geo g, PhaseArgs a) {
+__global__ void __launch_bounds__(kTileThreads, KIND == KIND_OR ? 9 : 7) phase64(Links64 L, RngStore R, Geo g, PhaseArgs a) {
   Nbr n;
   if (!tile_nbr<PAR>(g, n)) return;
   if (KIND != KIND_OR) count_draws(a);
@@ -45,9 +46,7 @@ __global__ void __launch_bounds__(kBlock) rng_setup(RngStore R, unsigned long lo
   __syncthreads();
   const int id = id0 + threadIdx.x;
   if (id >= vh) return;
-  curandStateMRG32k3a_t st;
-  mrg_jump_from(base, jumps, threadIdx.x, &st);
-  R.store(id, &st);
+  R.store(id, mrg_jump_from(base, jumps, threadIdx.x));
 }
 
 // ------------------------------------------------------------ starts -----
@@ -68,12 +67,12 @@ __global__ void __launch_bounds__(kBlock) init_cold(L links, int vh) {
 }
 
 // uniform cube (-0.5, 0.5]^4, normalised (su2_rand, su2.h:29-34)
-__device__ __forceinline__ Quat<double> random_link(curandStateMRG32k3a_t* st) {
+__device__ __forceinline__ Quat<double> random_link(MrgStream& st) {
   Quat<double> a;
-  a.w = curand_uniform_double(st) - 0.5;
-  a.x = curand_uniform_double(st) - 0.5;
-  a.y = curand_uniform_double(st) - 0.5;
-  a.z = curand_uniform_double(st) - 0.5;
+  a.w = st.uniform_double() - 0.5;
+  a.x = st.uniform_double() - 0.5;
+  a.y = st.uniform_double() - 0.5;
+  a.z = st.uniform_double() - 0.5;
   return q_normalize(a);
 }
 
@@ -85,8 +84,7 @@ template <class L>
 __global__ void __launch_bounds__(kBlock) init_hot(L links, RngStore R, Geo g, int pcc) {
   const int id = blockIdx.x * kBlock + threadIdx.x;
   if (id >= g.vh) return;
-  curandStateMRG32k3a_t st;
-  R.load(id, &st);
+  MrgStream st = R.load(id);
   for (int p = 0; p < 2; p++) {
     const Nbr n = make_nbr(g, id, p);
     const bool frozen = pcc && at_y0(g, n);
@@ -94,10 +92,10 @@ __global__ void __launch_bounds__(kBlock) init_hot(L links, RngStore R, Geo g, i
       if (d != DIR_Y && frozen)
         put(links, d, p, id, q_one<double>());
       else
-        put(links, d, p, id, random_link(&st));
+        put(links, d, p, id, random_link(st));
     }
   }
-  R.store(id, &st);
+  R.store(id, st);
 }
 
 // ------------------------------------------------------- re-projection --

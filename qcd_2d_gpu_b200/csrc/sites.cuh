@@ -3,7 +3,6 @@
 // checkerboard phase and the deterministic FP64 block reductions.  Templates
 // and inline functions only, so several translation units can include it.
 #pragma once
-#include <curand_kernel.h>
 #include "lattice.cuh"
 #include "rng.cuh"
 #include "su2.cuh"
@@ -77,20 +76,18 @@ __device__ __forceinline__ void site64(const Links64T<CG>& L, const RngStore& R,
   const int id = n.id;
   Quat<double> A = staple_sum<MU, BC, Links64T<CG>, double>(L, g, n, PAR);
   if (KIND == KIND_HB) {
-    curandStateMRG32k3a_t st;
-    R.load(id, &st);
-    Quat<double> U = heatbath_ref(A, (double)a.beta, &st, a.err);
+    MrgStream st = R.load(id);
+    Quat<double> U = heatbath_ref(A, (double)a.beta, st, a.err);
     if (!CG) chain_ready();
     L.st(MU, PAR, id, U);
-    R.store(id, &st);
+    R.store(id, st);
   } else if (KIND == KIND_METRO) {
-    curandStateMRG32k3a_t st;
-    R.load(id, &st);
+    MrgStream st = R.load(id);
     Quat<double> U = L.ld_own(MU, PAR, id);
-    int acc = metropolis_ref(U, A, (double)a.beta, (double)a.eps, a.upd, &st);
+    int acc = metropolis_ref(U, A, (double)a.beta, (double)a.eps, a.upd, st);
     if (!CG) chain_ready();
     L.st(MU, PAR, id, U);
-    R.store(id, &st);
+    R.store(id, st);
     atomicAdd(a.accept + PAR * g.vh + id, acc);
   } else {
     Quat<double> U = overrelax_ref(A, L.ld_own(MU, PAR, id));

@@ -13,7 +13,6 @@
 //        (mc_updates_pmc.h:33,40,96,103,156,163,219,225); the y links
 //        themselves use the periodic gather (mc_updates_pmc.h:250-251).
 #pragma once
-#include <curand_kernel.h>
 #include "lattice.cuh"
 #include "rng.cuh"
 #include "su2.cuh"
@@ -100,15 +99,15 @@ __device__ __forceinline__ Quat<R> staple_sum(const L& links, const Geo& g, cons
 // distribution, the new link built in double and normalised with rsqrt.
 // Returns the new link X A^+ with A the normalised staple.
 __device__ __forceinline__ Quat<double> heatbath_ref(Quat<double> A, double beta,
-                                                     curandStateMRG32k3a_t* st, int* err) {
+                                                     MrgStream& st, int* err) {
   double a;
   A = q_normalize_norm(A, &a);
   float inv = (float)(0.5 / (a * beta)), lf, aux;
   for (int tries = 1;; tries++) {
-    float r0 = curand_uniform(st), r1 = curand_uniform(st), r2 = curand_uniform(st);
+    float r0 = st.uniform(), r1 = st.uniform(), r2 = st.uniform();
     float c = cospif(2 * r1);
     lf = -(logf(r0) + c * c * logf(r2)) * inv;
-    aux = 1 - curand_uniform(st);
+    aux = 1 - st.uniform();
     if (!(aux * aux > 1 - lf)) break;
     if (tries >= QCD_HB_MAX_TRIES) {
       atomicOr(err, DEVERR_HB_LOOP);
@@ -118,8 +117,8 @@ __device__ __forceinline__ Quat<double> heatbath_ref(Quat<double> A, double beta
   Quat<double> X;
   X.w = 1 - 2 * (double)lf;
   double nrm = sqrt(1 - X.w * X.w);
-  float ct = 2 * curand_uniform(st) - 1, sp, cp;
-  sincospif(2 * curand_uniform(st), &sp, &cp);
+  float ct = 2 * st.uniform() - 1, sp, cp;
+  sincospif(2 * st.uniform(), &sp, &cp);
   float stt = sqrtf(fmaxf(0.f, 1 - ct * ct));
   double v1 = ct, v2 = (double)stt * cp, v3 = (double)stt * sp;
   double s = nrm * rsqrt(v1 * v1 + v2 * v2 + v3 * v3);
@@ -143,12 +142,12 @@ __device__ __forceinline__ bool metropolis_accept(double s, double u) {
 // `upd` Metropolis hits with proposals r U, r within eps of 1 (su2.h:87-97,
 // mc_updates.h:16-36, 119-128); A (not normalised) is reused by every hit.
 __device__ __forceinline__ int metropolis_ref(Quat<double>& U, const Quat<double>& A, double beta,
-                                              double eps, int upd, curandStateMRG32k3a_t* st) {
+                                              double eps, int upd, MrgStream& st) {
   int acc = 0;
   for (int h = 0; h < upd; h++) {
-    double r1 = curand_uniform_double(st) - 0.5;
-    double r2 = curand_uniform_double(st) - 0.5;
-    double r3 = curand_uniform_double(st) - 0.5;
+    double r1 = st.uniform_double() - 0.5;
+    double r2 = st.uniform_double() - 0.5;
+    double r3 = st.uniform_double() - 0.5;
     double nrm = sqrt(r1 * r1 + r2 * r2 + r3 * r3);
     Quat<double> r;
     r.x = eps * r1 / nrm;
@@ -158,7 +157,7 @@ __device__ __forceinline__ int metropolis_ref(Quat<double>& U, const Quat<double
     Quat<double> Un = q_mul(r, U);
     Quat<double> dU{Un.w - U.w, Un.x - U.x, Un.y - U.y, Un.z - U.z};
     double s = -beta * q_retr_mul(dU, A);
-    bool ok = s < 0 ? true : metropolis_accept(s, curand_uniform_double(st));
+    bool ok = s < 0 ? true : metropolis_accept(s, st.uniform_double());
     if (ok) {
       U = Un;
       acc++;
