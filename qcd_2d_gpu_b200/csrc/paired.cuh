@@ -223,8 +223,7 @@ __device__ __forceinline__ Q2 p2_mul_bd_first(const Q2& a, const Q2& b) {
 }
 // T: a t phase, whose |A|^2 starts from the other term: the rounding with which
 // chains of these phases have always run, so that a seed keeps its chain.
-template <bool T>
-__device__ __forceinline__ Q2 heatbath2(Q2 A, const PhaseArgs& a, uint32_t site0, uint32_t site1) {
+__device__ __forceinline__ Q2 heatbath2(Q2 A, const PhaseArgs& a, uint32_t site0, uint32_t site1, bool T) {
   const unsigned long long phase = draw_phase(a);
   const float2 wx = T ? fma2(A.w, A.w, mul2(A.x, A.x)) : fma2(A.x, A.x, mul2(A.w, A.w));
   const float2 det = fma2(A.z, A.z, fma2(A.y, A.y, wx));
@@ -276,30 +275,29 @@ __device__ __forceinline__ Q2 heatbath2(Q2 A, const PhaseArgs& a, uint32_t site0
 }
 
 // ------------------------------------------------------------ one phase --
-// The new links of both lanes of pair n (sublattice PAR); gid0 is lane 0's
-// sublattice index (lane 1's is gid0 + V/4), used for the counter-based
-// draws and the Metropolis accept counters.
-template <int MU, int PAR, int BC, int KIND, class PS>
-__device__ __forceinline__ Q2 pair_update(const PS& P, const Geo& gh, const PhaseArgs& a, const Nbr& n, bool sp,
-                                          bool sm, int renorm) {
-  const Q2 A = staple_sum2<MU, BC>(P, gh, n, PAR, sp, sm);
-  const unsigned int gid0 = (unsigned int)n.id, gid1 = gid0 + (unsigned int)P.vhp;
+// The new links of both lanes of pair `id` of link class (mu, par) from their
+// staple sums; id is lane 0's sublattice index (lane 1's is id + V/4), used for the
+// counter-based draws and the Metropolis accept counters.
+template <int KIND, class PS>
+__device__ __forceinline__ Q2 pair_new(const PS& P, const Q2& A, const PhaseArgs& a, int mu, int par, int id,
+                                       int renorm) {
+  const unsigned int gid0 = (unsigned int)id, gid1 = gid0 + (unsigned int)P.vhp;
   Q2 U;
   if (KIND == KIND_HB) {
-    U = heatbath2<MU == DIR_T>(A, a, a.site_off + gid0, a.site_off + gid1);
+    U = heatbath2(A, a, a.site_off + gid0, a.site_off + gid1, mu == DIR_T);
   } else if (KIND == KIND_METRO) {
-    const Q2 U0 = P.ld_own(MU, PAR, n.id);
+    const Q2 U0 = P.ld_own(mu, par, id);
     Quat<float> u0 = lane0(U0), u1 = lane1(U0);
     PhiloxStream s0(a.keys, a.site_off + gid0, draw_phase(a));
     PhiloxStream s1(a.keys, a.site_off + gid1, draw_phase(a));
     const int acc0 = metropolis_fast(u0, lane0(A), a.beta, a.eps, a.upd, s0);
     const int acc1 = metropolis_fast(u1, lane1(A), a.beta, a.eps, a.upd, s1);
-    int* acc = a.accept + PAR * 2 * P.vhp;
+    int* acc = a.accept + par * 2 * P.vhp;
     atomicAdd(acc + gid0, acc0);
     atomicAdd(acc + gid1, acc1);
     U = join(u0, u1);
   } else {
-    U = overrelax2(A, P.ld_own(MU, PAR, n.id));
+    U = overrelax2(A, P.ld_own(mu, par, id));
   }
   if (renorm) U = join(renorm_fast(lane0(U)), renorm_fast(lane1(U)));
   return U;
@@ -314,7 +312,8 @@ __global__ void __launch_bounds__(kTileThreads, 8) phase32p(Pair32 P, Geo gh, Ph
   if (!tile_nbr<PAR>(gh, n)) return;
   if (KIND != KIND_OR) count_draws(a);
   if (BC == BC_PCC && MU != DIR_Y && at_y0(gh, n)) return;
-  const Q2 U = pair_update<MU, PAR, BC, KIND>(P, gh, a, n, n.t == gh.lt - 1, n.t == 0, a.renorm);
+  const Q2 A = staple_sum2<MU, BC>(P, gh, n, PAR, n.t == gh.lt - 1, n.t == 0);
+  const Q2 U = pair_new<KIND>(P, A, a, MU, PAR, n.id, a.renorm);
   chain_ready();
   P.st(MU, PAR, n.id, U);
 }

@@ -116,7 +116,7 @@ cudaError_t pair_pass32(const float4* cur, float4* alt, const PairMaps& maps_cur
     pg.seg = seg > 0 ? (seg < ls ? seg : ls) : pair_segment(ls, tiles, sms);
     const dim3 grid((unsigned int)tiles, (unsigned int)((ls + pg.seg - 1) / pg.seg));
     PhaseArgs am = a;
-    am.phase_off = a.phase_off + (unsigned int)(2 * mu);
+    am.phase_off = a.phase_off + 2 * mu;
     void* fn = pick(mu, bc, kind);
     const int slot = mu * 9 + bc * 3 + (kind == KIND_HB ? 1 : kind == KIND_METRO ? 0 : 2);
     cudaError_t e = opt_in(fn, slot);

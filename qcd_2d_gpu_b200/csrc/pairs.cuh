@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(PairCfg<MU>::NT, 1)
   const bool in_tile_1 = C::YRING ? (w_1 >= C::W0 && w_1 < C::W0 + ny) : tile_row;
   const int row_off = r * kPairW;
   PhaseArgs ap = a;
-  ap.phase_off = a.phase_off + (unsigned int)par;
+  ap.phase_off = a.phase_off + par;
 
   const int J = s1 - s0 + 3;
   for (int j = 0; j < J; j++) {

@@ -16,6 +16,7 @@
 #include "paired.cuh"
 #include "pairs.h"
 #include "qcd2d.h"
+#include "resident.cuh"
 #include "wave.cuh"
 
 using namespace qcd;
@@ -73,6 +74,7 @@ struct qcd_lattice {
   int wave_tasks_chunk[5] = {0, 0, 0, 0, 0};
   int wave_tasks_fronts[5] = {0, 0, 0, 0, 0};
   int sms = 0;       // multiprocessors of the device (fused pairs)
+  int resident_can[2] = {-1, -1};  // small lattices: one cluster can hold the passes (planes, pairs; -1: not asked)
   // fused pairs: the two FP32 stores and their tensor maps (pair_buf[0] is
   // the store allocated at create; q32 / q32alt point at one each)
   float4* pair_buf[2] = {nullptr, nullptr};
@@ -490,6 +492,73 @@ bool use_wave(const qcd_lattice* h) {
 
 bool use_pairs(const qcd_lattice* h) { return h->sched == QCD_SCHED_PAIRS && h->p.precision == QCD_PREC_FP32; }
 
+// ------------------------------------------------------------- resident --
+// The launch of up to kResidentPasses passes in one cluster (resident.cuh); with
+// `probe` nothing is launched and the kernel is only asked whether this device
+// can run such a cluster.
+template <class S>
+cudaError_t launch_resident(const qcd_lattice* h, S L, typename S::Global global, const Geo& g, const PhaseArgs& a,
+                            const ResidentProgram& p, bool probe) {
+  auto fn = h->p.algo == QCD_ALGO_HEATBATH ? resident<S, KIND_HB> : resident<S, KIND_METRO>;
+  L.m.lg = 5;
+  while ((kResidentCtas << L.m.lg) < g.vh) L.m.lg++;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(kResidentCtas);
+  c.blockDim = dim3(1u << L.m.lg);
+  c.dynamicSmemBytes = (size_t)resident_bytes<S>(L.m.lg);
+  c.stream = h->stream;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kResidentCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 2;
+  if (!probe) return cudaLaunchKernelEx(&c, fn, L, global, rngs(h), g, a, p, h->p.boundary, h->draw_dev);
+  c.numAttrs = 1;
+  int clusters = 0;
+  cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_bytes<S>(kResidentLog));
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (const void*)fn, &c);
+  return e != cudaSuccess ? e : clusters > 0 ? cudaSuccess : cudaErrorNotSupported;
+}
+
+cudaError_t resident_call(const qcd_lattice* h, const ResidentProgram& p, bool probe) {
+  PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, 0, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
+  if (h->paired) return launch_resident(h, ClusterPair{{}, h->gh.vh}, pair32(h), h->gh, a, p, probe);
+  if (h->p.precision == QCD_PREC_FP64) return launch_resident(h, Cluster64{}, links64(h), h->g, a, p, probe);
+  return launch_resident(h, Cluster32{}, links32(h), h->g, a, p, probe);
+}
+
+// Whether the per-phase schedule runs this lattice's passes in one cluster (asked
+// of the device once per store layout).
+bool use_resident(qcd_lattice* h) {
+  const bool planes32 = h->p.precision == QCD_PREC_FP32 && !h->paired;
+  if ((h->paired ? h->gh.vh : h->g.vh) > (planes32 ? kResidentItems32 : kResidentItems)) return false;
+  int& can = h->resident_can[h->paired];
+  if (can < 0) {
+    can = resident_call(h, ResidentProgram{}, true) == cudaSuccess;
+    if (!can) cudaGetLastError();
+  }
+  return can > 0;
+}
+
+// up to kResidentPasses passes of a small lattice in one launch
+int pass_resident(qcd_lattice* h, const PassSpec* ps, int np) {
+  ResidentProgram p;
+  p.n = np;
+  for (int i = 0; i < np; i++) {
+    p.kind[i] = (unsigned char)ps[i].kind;
+    p.renorm[i] = (unsigned char)ps[i].renorm;
+  }
+  CUDA_OR_FAIL(h, resident_call(h, p, false));
+  for (int i = 0; i < np; i++)
+    if (ps[i].kind != KIND_METRO) h->unit_passes++;
+  return QCD_OK;
+}
+
 // The second store and the device facts the fused pairs need (allocated
 // when the schedule is chosen, never inside a pass, so that passes can be
 // captured in a CUDA graph).
@@ -616,6 +685,13 @@ int run_passes(qcd_lattice* h, const PassSpec* ps, int np) {
     for (int i = 0; i < np; i += h->wave_chain) {
       const int k = np - i < h->wave_chain ? np - i : h->wave_chain;
       rc = launch_wave(h, ps + i, k);
+      if (rc) return rc;
+    }
+    return QCD_OK;
+  }
+  if (use_resident(h)) {
+    for (int i = 0; i < np; i += kResidentPasses) {
+      int rc = pass_resident(h, ps + i, std::min(np - i, kResidentPasses));
       if (rc) return rc;
     }
     return QCD_OK;

@@ -24,8 +24,8 @@ struct PhaseArgs {
   // every replay), this phase's offset from it, and the offset added to the
   // site index (a replica's stream offset in a batch)
   unsigned long long seed;
-  const unsigned long long* phase_ptr;
-  int phase_off;
+  const unsigned long long* phase_ptr;  // null: phase_off is the number itself
+  long long phase_off;
   unsigned int site_off;
   PhiloxKeys keys;  // round keys of `seed` (philox_keys), set by whoever fills the arguments
   // where this launch writes the count for later launches (count_draws), or null
@@ -56,7 +56,7 @@ __device__ __forceinline__ void count_draws(const PhaseArgs& a) {
 }
 // the drawing-phase number of this launch
 __device__ __forceinline__ unsigned long long draw_phase(const PhaseArgs& a) {
-  return draw_count(a) + (long long)a.phase_off;
+  return (a.phase_ptr ? draw_count(a) : 0) + a.phase_off;
 }
 
 // The wavefront and the fused pairs, which read word 0 alone, advance it by this
@@ -99,51 +99,43 @@ __device__ __forceinline__ void site64(const Links64T<CG>& L, const RngStore& R,
 // FP32: the same updates with FP32 links and FP64 fix-ups; the heat-bath and
 // Metropolis draw from the counter-based Philox stream of (site, phase), so
 // no generator state is read or written.
-// The new value of FP32 link U_MU at a site of sublattice PAR whose global
-// sublattice index is gid (the Philox site counter and the accept slot);
-// `links` and `n` address the staple links (global memory here, a
-// shared-memory tile in the fused-pair kernel).  Metropolis accept counts are
-// added only when count_accept is set.
-template <int MU, int PAR, int BC, int KIND, class L>
-__device__ __forceinline__ Quat<float> link_update32(const L& links, const Geo& g, const PhaseArgs& a, const Nbr& n,
-                                                     int gid, int renorm, bool count_accept) {
-  Quat<float> A = staple_sum<MU, BC, L, float>(links, g, n, PAR);
+// The new value of FP32 link U_mu of site `id` of sublattice `par` from its staple
+// sum; gid is the site's global sublattice index (the Philox site counter and
+// the accept slot), `links` and `id` address the link's store.  Metropolis
+// accept counts are added only when count_accept is set.
+template <int KIND, class L>
+__device__ __forceinline__ Quat<float> link_new32(const L& links, const Quat<float>& A, const Geo& g,
+                                                  const PhaseArgs& a, int mu, int par, int id, int gid, int renorm,
+                                                  bool count_accept) {
   Quat<float> U;
   if (KIND == KIND_HB) {
     PhiloxStream st(a.keys, a.site_off + (unsigned int)gid, draw_phase(a));
     U = heatbath_fast(A, a.beta, st, a.err);
   } else if (KIND == KIND_METRO) {
     PhiloxStream st(a.keys, a.site_off + (unsigned int)gid, draw_phase(a));
-    U = links.ld_own(MU, PAR, n.id);
+    U = links.ld_own(mu, par, id);
     int acc = metropolis_fast(U, A, a.beta, a.eps, a.upd, st);
-    if (count_accept) atomicAdd(a.accept + PAR * g.vh + gid, acc);
+    if (count_accept) atomicAdd(a.accept + par * g.vh + gid, acc);
   } else {
-    U = overrelax_fast(A, links.ld_own(MU, PAR, n.id));
+    U = overrelax_fast(A, links.ld_own(mu, par, id));
   }
   return renorm ? renorm_fast(U) : U;
+}
+// the same with the staples gathered at n (a shared-memory tile in the fused-pair kernel)
+template <int MU, int PAR, int BC, int KIND, class L>
+__device__ __forceinline__ Quat<float> link_update32(const L& links, const Geo& g, const PhaseArgs& a, const Nbr& n,
+                                                     int gid, int renorm, bool count_accept) {
+  const Quat<float> A = staple_sum<MU, BC, L, float>(links, g, n, PAR);
+  return link_new32<KIND>(links, A, g, a, MU, PAR, n.id, gid, renorm, count_accept);
 }
 
 template <int MU, int PAR, int BC, int KIND, bool CG>
 __device__ __forceinline__ void site32(const Links32T<CG>& L, const RngStore& R, const Geo& g,
                                        const PhaseArgs& a, const Nbr& n, int renorm) {
   if (BC == BC_PCC && MU != DIR_Y && at_y0(g, n)) return;
-  const int id = n.id;
-  Quat<float> A = staple_sum<MU, BC, Links32T<CG>, float>(L, g, n, PAR);
-  Quat<float> U;
-  if (KIND == KIND_HB) {
-    PhiloxStream st(a.keys, a.site_off + (unsigned int)id, draw_phase(a));
-    U = heatbath_fast(A, a.beta, st, a.err);
-  } else if (KIND == KIND_METRO) {
-    PhiloxStream st(a.keys, a.site_off + (unsigned int)id, draw_phase(a));
-    U = L.ld_own(MU, PAR, id);
-    int acc = metropolis_fast(U, A, a.beta, a.eps, a.upd, st);
-    atomicAdd(a.accept + PAR * g.vh + id, acc);
-  } else {
-    U = overrelax_fast(A, L.ld_own(MU, PAR, id));
-  }
-  if (renorm) U = renorm_fast(U);
+  const Quat<float> U = link_update32<MU, PAR, BC, KIND>(L, g, a, n, n.id, renorm, true);
   if (!CG) chain_ready();
-  L.st(MU, PAR, id, U);
+  L.st(MU, PAR, n.id, U);
 }
 
 // ---------------------------------------------------------- reductions --
