@@ -300,7 +300,7 @@ int qcd_batch_reserve(qcd_batch* b, int capacity);
 int qcd_batch_run(qcd_batch* b, int sweeps, int measure_every, int use_graph);
 /* Groups: the replicas are swept in groups of consecutive replicas holding
    at most bytes_per_group bytes of links (at least one replica each; 0: one
-   group of everything; default 32 MB), each group going through all the
+   group of everything; default 16 MB, FP64 24 MB), each group going through all the
    sweeps of a qcd_batch_run while its links stay in L2 before the next group
    starts.  Replicas are independent and every group keeps its own
    drawing-phase counter and measurement cursor, so the results do not depend
@@ -308,7 +308,7 @@ int qcd_batch_run(qcd_batch* b, int sweeps, int measure_every, int use_graph);
 int qcd_batch_set_groups(qcd_batch* b, long long bytes_per_group);
 /* number of groups */
 int qcd_batch_groups(const qcd_batch* b);
-/* Lanes (1..4, default 2): streams on which groups run at the same time,
+/* Lanes (1..4, default 4, FP64 3): streams on which groups run at the same time,
    group g on lane g mod lanes, forked from and joined back into the batch's
    stream; one group's memory-bound measurement then overlaps another's
    phases. */

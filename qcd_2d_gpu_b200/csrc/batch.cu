@@ -72,8 +72,12 @@ struct BatchArgs {
   unsigned int count_add;
 };
 
+// CTAs per SM, measured on 96 mixed replicas (20 heat-bath sweeps): FP32 five, 19.1 ms
+// (19.3 at six, 19.8 at four, 22.1 at three); FP64 four, 37.6 ms (43.4 at six, 38.5 at
+// five, 38.3 at three).  Tiles as in the lone phases gain nothing here: the replicas
+// of a group lie in L2, and a tile's CTA looks up its replica for half as many sites.
 template <int MU, int PAR, int KIND, bool FP64>
-__global__ void __launch_bounds__(kBlock, 6) batch_phase(BatchView B, BatchArgs a) {
+__global__ void __launch_bounds__(kBlock, FP64 ? 4 : 5) batch_phase(BatchView B, BatchArgs a) {
   const int cta = batch_cta(B);
   const int r = replica_of(B, cta);
   const Replica& R = B.rep[r];
@@ -258,10 +262,13 @@ BatchPhaseFn batch_phase_fn(int k, int kind) {
 // links stay in L2 before the next group starts (each group with its own
 // drawing-phase counter and measurement cursor, so every replica draws and
 // records exactly what it would in one group of everything).
-// default grouping (the autotuner's choice for 96 mixed replicas, C4): groups
-// of up to 32 MB of links, well inside the 126 MB L2, two at a time
-constexpr long long kBatchGroupBytes = 32ll << 20;
-constexpr int kBatchLanes = 2;
+// Default grouping, well inside the 126 MB L2 and the best or within 3% of it over
+// batches of 10 to 96 mixed replicas: FP32 four groups of 16 MB at a time (96, 40, 20
+// and 10 replicas up to 64 x 64 x 128: 20 sweeps 19.0, 7.71, 3.37 and 1.71 ms against
+// 19.1, 7.97, 3.54 and 1.77 ms with two of 32 MB), FP64 three of 24 MB (96, 30 and 80
+// replicas: 38.5, 4.64 and 1.66 ms against 37.6, 5.22 and 1.84 ms).
+constexpr long long kBatchGroupBytes32 = 16ll << 20, kBatchGroupBytes64 = 24ll << 20;
+constexpr int kBatchLanes32 = 4, kBatchLanes64 = 3;
 
 struct BatchGroup {
   int r0, r1;         // replicas [r0, r1)
@@ -304,7 +311,7 @@ struct qcd_batch {
   // lanes: streams that run groups concurrently (group g on lane g mod lanes),
   // forked from and joined back into `stream` by events
   static constexpr int kMaxLanes = 4;
-  int lanes = kBatchLanes;
+  int lanes = kBatchLanes32;
   cudaStream_t lane[kMaxLanes] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t fork_ev = nullptr, join_ev[kMaxLanes] = {nullptr, nullptr, nullptr, nullptr};
   int graph_every = 0;
@@ -581,7 +588,8 @@ int qcd_batch_create(const qcd_replica* r, int n, const qcd_params* common, qcd_
     delete b;
     return rc;
   }
-  form_groups(b, kBatchGroupBytes);
+  b->lanes = fp64(b) ? kBatchLanes64 : kBatchLanes32;
+  form_groups(b, fp64(b) ? kBatchGroupBytes64 : kBatchGroupBytes32);
   *out = b;
   return QCD_OK;
 }

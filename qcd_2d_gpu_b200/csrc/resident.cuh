@@ -196,24 +196,24 @@ __device__ __forceinline__ void resident_update(const Cluster64& L, uint32_t* rn
   const Quat<double> A = resident_staples(L, g, n, mu, par, bc, false);
   if (KIND == KIND_OR) {
     L.st(mu, par, n.id, overrelax_ref(A, L.ld_own(mu, par, n.id)));
-    return;
-  }
-  MrgStream st;
-  for (int i = 0; i < 3; i++) {
-    st.s1[i] = rng[i * step + l];
-    st.s2[i] = rng[(3 + i) * step + l];
-  }
-  if (KIND == KIND_HB) {
-    L.st(mu, par, n.id, heatbath_ref(A, (double)a.beta, st, a.err));
   } else {
-    Quat<double> U = L.ld_own(mu, par, n.id);
-    const int acc = metropolis_ref(U, A, (double)a.beta, (double)a.eps, a.upd, st);
-    L.st(mu, par, n.id, U);
-    atomicAdd(a.accept + par * g.vh + n.id, acc);
-  }
-  for (int i = 0; i < 3; i++) {
-    rng[i * step + l] = st.s1[i];
-    rng[(3 + i) * step + l] = st.s2[i];
+    MrgStream st;
+    for (int i = 0; i < 3; i++) {
+      st.s1[i] = rng[i * step + l];
+      st.s2[i] = rng[(3 + i) * step + l];
+    }
+    if (KIND == KIND_HB) {
+      L.st(mu, par, n.id, heatbath_ref(A, (double)a.beta, st, a.err));
+    } else {
+      Quat<double> U = L.ld_own(mu, par, n.id);
+      const int acc = metropolis_ref(U, A, (double)a.beta, (double)a.eps, a.upd, st);
+      L.st(mu, par, n.id, U);
+      atomicAdd(a.accept + par * g.vh + n.id, acc);
+    }
+    for (int i = 0; i < 3; i++) {
+      rng[i * step + l] = st.s1[i];
+      rng[(3 + i) * step + l] = st.s2[i];
+    }
   }
 }
 template <int KIND>
