@@ -270,6 +270,8 @@ BatchPhaseFn batch_phase_fn(int k, int kind) {
 constexpr long long kBatchGroupBytes32 = 16ll << 20, kBatchGroupBytes64 = 24ll << 20;
 constexpr int kBatchLanes32 = 4, kBatchLanes64 = 3;
 
+constexpr int kBatchStage = 1024;
+
 struct BatchGroup {
   int r0, r1;         // replicas [r0, r1)
   int cta0, ctas;     // its CTAs in the phase launches' table
@@ -305,6 +307,9 @@ struct qcd_batch {
   unsigned int* rep_count = nullptr;
   double2* series = nullptr;
   int cap = 0;
+  // pinned staging of what the host reads back: kBatchStage pairs of a series, then
+  // the device error word
+  double2* stage = nullptr;
   long long sweeps_done = 0;
   std::vector<BatchGroup> groups;
   long long group_bytes = 0;  // target link bytes per group (0: one group)
@@ -457,6 +462,7 @@ void release(qcd_batch* b) {
   cudaFree(b->all_count);
   cudaFree(b->cursor);
   cudaFree(b->series);
+  if (b->stage) cudaFreeHost(b->stage);
   for (int k = 0; k < qcd_batch::kMaxLanes; k++) {
     if (b->lane[k]) cudaStreamDestroy(b->lane[k]);
     if (b->join_ev[k]) cudaEventDestroy(b->join_ev[k]);
@@ -570,6 +576,7 @@ int qcd_batch_create(const qcd_replica* r, int n, const qcd_params* common, qcd_
     if (rc == QCD_OK) step(cudaMemsetAsync(b->accept, 0, site_off * sizeof(int), b->stream), "memset");
   }
   if (rc == QCD_OK) step(cudaMalloc(&b->err, sizeof(int)), "cudaMalloc(err)");
+  if (rc == QCD_OK) step(cudaMallocHost(&b->stage, (kBatchStage + 1) * sizeof(double2)), "cudaMallocHost");
   if (rc == QCD_OK) step(cudaMalloc(&b->draw_dev, 2 * n * sizeof(unsigned long long)), "cudaMalloc(draw counters)");
   if (rc == QCD_OK) step(cudaMemsetAsync(b->draw_dev, 0, n * sizeof(unsigned long long), b->stream), "memset");
   if (rc == QCD_OK)
@@ -863,8 +870,9 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
 int qcd_batch_synchronize(qcd_batch* b) {
   if (!b) return QCD_ERR_INVALID;
   int e = 0;
-  BCUDA(b, cudaMemcpyAsync(&e, b->err, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+  BCUDA(b, cudaMemcpyAsync(b->stage + kBatchStage, b->err, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));
+  memcpy(&e, b->stage + kBatchStage, sizeof(int));
   if (e & DEVERR_HB_LOOP)
     return bfail(b, QCD_ERR_NONUNITARY, "heat-bath rejection loop exceeded %d tries", QCD_HB_MAX_TRIES);
   return QCD_OK;
@@ -880,14 +888,19 @@ int qcd_batch_measured(qcd_batch* b) {
 
 int qcd_batch_series(qcd_batch* b, int replica, double* energy, double* plaquette, int n) {
   if (!b || replica < 0 || replica >= b->n || n < 0 || n > b->cap) return QCD_ERR_INVALID;
-  int rc = qcd_batch_synchronize(b);
-  if (rc) return rc;
-  if (n == 0) return QCD_OK;
-  std::vector<double2> tmp(n);
-  BCUDA(b, cudaMemcpy(tmp.data(), b->series + (size_t)replica * b->cap, n * sizeof(double2), cudaMemcpyDeviceToHost));
-  for (int i = 0; i < n; i++) {
-    if (energy) energy[i] = tmp[i].x;
-    if (plaquette) plaquette[i] = tmp[i].y;
+  // the first pairs and the error word come with one wait (a read per replica is what
+  // a program does after a run: 96 of them 2.8 ms with a wait for each and pageable copies)
+  for (int i0 = 0; i0 == 0 || i0 < n; i0 += kBatchStage) {
+    const int m = n - i0 < kBatchStage ? n - i0 : kBatchStage;
+    if (m > 0)
+      BCUDA(b, cudaMemcpyAsync(b->stage, b->series + (size_t)replica * b->cap + i0, m * sizeof(double2),
+                               cudaMemcpyDeviceToHost, b->stream));
+    int rc = qcd_batch_synchronize(b);
+    if (rc) return rc;
+    for (int i = 0; i < m; i++) {
+      if (energy) energy[i0 + i] = b->stage[i].x;
+      if (plaquette) plaquette[i0 + i] = b->stage[i].y;
+    }
   }
   return QCD_OK;
 }
