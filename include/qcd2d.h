@@ -153,9 +153,9 @@ int qcd_check_unitarity(qcd_lattice* h, double tol, double* mean_det);
  * Scheduling of the six checkerboard phases (replaces the reference's six
  * serial launches per sweep, mc_updates.h:467-475, with the same result).
  *   PHASES     one launch per phase: each phase streams the link store.  The
- *              passes of a small lattice (up to 2048 sites of a parity or site
- *              pairs, 4096 sites of FP32 planes) run in one launch of one
- *              thread-block cluster instead, with the same result.
+ *              passes of a small lattice (up to 4096 sites of a parity or site
+ *              pairs; Metropolis 2048, but 4096 on FP32 planes) run in one launch
+ *              of one thread-block cluster instead, with the same result.
  *   WAVEFRONT  one persistent launch per chain of passes: every t-slice goes
  *              through the phases of the chain while it is resident in L2;
  *              tasks run in a ring schedule ordered so that each waits only

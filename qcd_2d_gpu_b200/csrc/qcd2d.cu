@@ -536,7 +536,8 @@ cudaError_t resident_call(const qcd_lattice* h, const ResidentProgram& p, bool p
 // of the device once per store layout).
 bool use_resident(qcd_lattice* h) {
   const bool planes32 = h->p.precision == QCD_PREC_FP32 && !h->paired;
-  if ((h->paired ? h->gh.vh : h->g.vh) > (planes32 ? kResidentItems32 : kResidentItems)) return false;
+  const int most = h->p.algo == QCD_ALGO_METROPOLIS && !planes32 ? kResidentItemsMetro : kResidentItems;
+  if ((h->paired ? h->gh.vh : h->g.vh) > most) return false;
   int& can = h->resident_can[h->paired];
   if (can < 0) {
     can = resident_call(h, ResidentProgram{}, true) == cudaSuccess;

@@ -24,13 +24,14 @@ namespace qcd {
 constexpr int kResidentCtas = 16;
 constexpr int kResidentLog = 8;  // most slots of a CTA: 2^8, one thread each
 constexpr int kResidentPasses = 64;
-// Largest work of a phase (sites; pairs) for which one cluster is faster than
-// launches on the whole GPU: at 4000 FP64 sites the two are level (100 us for five
-// heat-bath sweeps), at 3360 pairs the launches lead (64 against 68 us for 24
-// phases); a site of a single-precision plane has half the bytes to fetch (7260
-// sites: 62 against 58 us, Metropolis level).
-constexpr int kResidentItems = 2048, kResidentItems32 = 4096;
-static_assert(kResidentItems32 <= kResidentCtas << kResidentLog, "slots for every site");
+// Largest work of a phase (sites; pairs) for which one cluster is faster than launches
+// on the whole GPU: heat-bath and over-relaxation 4096 (4000 FP64 sites: five
+// heat-bath sweeps 97 against 100 us; 3360 pairs: 24 phases 64 against 64-77 us,
+// 2048 pairs 44 against 60), Metropolis, whose hits are longer, 2048 (3360 pairs: 218
+// against 205 us) but on single-precision planes, whose sites have half the bytes to
+// fetch (3960 sites: level).
+constexpr int kResidentItems = 4096, kResidentItemsMetro = 2048;
+static_assert(kResidentItems <= kResidentCtas << kResidentLog, "slots for every site");
 
 struct ResidentProgram {
   int n;  // passes

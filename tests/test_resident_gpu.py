@@ -1,6 +1,6 @@
 """Small lattices, whose passes run in one cluster (links in shared memory), around
-the sizes where that begins and ends: up to 2048 sites of a parity (FP64) or site
-pairs, 4096 sites of FP32 planes.  Exact comparisons."""
+the sizes where that begins and ends: up to 4096 sites of a parity or site pairs
+(Metropolis 2048, but 4096 on FP32 planes).  Exact comparisons."""
 import numpy as np
 import pytest
 
@@ -31,7 +31,7 @@ def test_cluster_equals_the_wavefront(dims, bc, prec, algo):
         assert np.array_equal(x, y)
 
 
-@pytest.mark.parametrize("dims", [(4, 2, 2), (8, 6, 10), (16, 16, 32), (16, 18, 30)], ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("dims", [(4, 2, 2), (8, 6, 10), (16, 16, 32), (16, 18, 30), (16, 32, 32), (16, 30, 36)], ids=lambda d: "x".join(map(str, d)))
 @pytest.mark.parametrize("algo", ["hb", "metro"])
 def test_pairs_do_not_depend_on_the_split_into_launches(dims, algo):
     # 84 passes in one call (more than a launch takes) and in 21 calls
