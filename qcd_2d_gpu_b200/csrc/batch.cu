@@ -34,7 +34,7 @@ struct Replica {
   float beta;
   int bc;
   int hot;
-  long long link_off;  // float4 units (FP32) or double2 units per lo/hi plane (FP64)
+  long long link_off;  // links before this replica
   long long rng_off;   // u32 words
   long long site_off;  // accept counters
   int cta_begin;       // first CTA of this replica in a batched launch
@@ -50,8 +50,7 @@ struct BatchView {
   int n;               // replicas the launch covers
   int cta0, mcta0;     // first CTA of the launch in the batch's CTA tables (a group's offset)
   float4* q32;
-  double2* lo;
-  double2* hi;
+  double* q64;
   uint32_t* rng;
 };
 
@@ -93,7 +92,7 @@ __global__ void __launch_bounds__(kBlock, FP64 ? 4 : 5) batch_phase(BatchView B,
   if (KIND != KIND_OR) count_draws(pa);
   RngStore RS{B.rng + R.rng_off, R.g.vh};
   if (FP64) {
-    Links64 L{B.lo + R.link_off, B.hi + R.link_off, R.g.vh};
+    Links64 L{B.q64 + 4 * R.link_off, R.g.vh};
     switch (R.bc) {
       case BC_PER: site64<MU, PAR, BC_PER, KIND, false>(L, RS, R.g, pa, n); break;
       case BC_PCC: site64<MU, PAR, BC_PCC, KIND, false>(L, RS, R.g, pa, n); break;
@@ -137,7 +136,7 @@ __global__ void __launch_bounds__(kBlock) batch_setup(BatchView B, const uint32_
         u = q_normalize(u);
       }
       if (FP64) {
-        Links64 L{B.lo + R.link_off, B.hi + R.link_off, R.g.vh};
+        Links64 L{B.q64 + 4 * R.link_off, R.g.vh};
         L.st(d, p, id, u);
       } else {
         Links32 L{B.q32 + R.link_off, R.g.vh};
@@ -159,7 +158,7 @@ __global__ void __launch_bounds__(kBlock) batch_normalize(BatchView B) {
   for (int p = 0; p < 2; p++)
     for (int d = 0; d < 3; d++) {
       if (FP64) {
-        Links64 L{B.lo + R.link_off, B.hi + R.link_off, R.g.vh};
+        Links64 L{B.q64 + 4 * R.link_off, R.g.vh};
         L.st(d, p, id, q_normalize(L.ld_own(d, p, id)));
       } else {
         Links32 L{B.q32 + R.link_off, R.g.vh};
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(kBlock, FP64 ? kMeasurePerSM64 : kMeasurePerSM
   const int nblk = (int)measure_blocks(R.g.vh, FP64 ? kMeasurePerSM64 : kMeasurePerSM32);
   double e = 0, pl = 0;
   if (FP64) {
-    Links64 L{B.lo + R.link_off, B.hi + R.link_off, R.g.vh};
+    Links64 L{B.q64 + 4 * R.link_off, R.g.vh};
     if (R.bc == BC_PMC)
       measure_sites<Links64, true>(L, R.g, mcta - R.mcta_begin, nblk, e, pl);
     else
@@ -291,8 +290,7 @@ struct qcd_batch {
   int* mcta_rep = nullptr;
   int mctas = 0;
   float4* q32 = nullptr;
-  double2* lo = nullptr;
-  double2* hi = nullptr;
+  double* q64 = nullptr;
   uint32_t* rng = nullptr;
   uint32_t* mrg_jumps = nullptr;  // jump matrices that seed the streams (mrg_jump_table)
   // per group (n entries, groups use the first ones): drawing phases run so
@@ -347,11 +345,11 @@ int bfail(qcd_batch* b, int code, const char* fmt, ...) {
 
 // every replica (setup, whole-batch launches)
 BatchView view(const qcd_batch* b) {
-  return BatchView{b->rep_dev, b->cta_rep, b->mcta_rep, b->n, 0, 0, b->q32, b->lo, b->hi, b->rng};
+  return BatchView{b->rep_dev, b->cta_rep, b->mcta_rep, b->n, 0, 0, b->q32, b->q64, b->rng};
 }
 // the replicas of one group
 BatchView view(const qcd_batch* b, const BatchGroup& g) {
-  return BatchView{b->rep_dev, b->cta_rep, b->mcta_rep, g.r1 - g.r0, g.cta0, g.mcta0, b->q32, b->lo, b->hi, b->rng};
+  return BatchView{b->rep_dev, b->cta_rep, b->mcta_rep, g.r1 - g.r0, g.cta0, g.mcta0, b->q32, b->q64, b->rng};
 }
 
 bool fp64(const qcd_batch* b) { return b->common.precision == QCD_PREC_FP64; }
@@ -450,8 +448,7 @@ void release(qcd_batch* b) {
   cudaFree(b->cta_rep);
   cudaFree(b->mcta_rep);
   cudaFree(b->q32);
-  cudaFree(b->lo);
-  cudaFree(b->hi);
+  cudaFree(b->q64);
   cudaFree(b->rng);
   cudaFree(b->mrg_jumps);
   cudaFree(b->accept);
@@ -561,8 +558,7 @@ int qcd_batch_create(const qcd_replica* r, int n, const qcd_params* common, qcd_
            "cta table");
   }
   if (common->precision == QCD_PREC_FP64) {
-    if (rc == QCD_OK) step(cudaMalloc(&b->lo, link_off * sizeof(double2)), "cudaMalloc(links)");
-    if (rc == QCD_OK) step(cudaMalloc(&b->hi, link_off * sizeof(double2)), "cudaMalloc(links)");
+    if (rc == QCD_OK) step(cudaMalloc(&b->q64, link_off * 4 * sizeof(double)), "cudaMalloc(links)");
   } else if (rc == QCD_OK) {
     step(cudaMalloc(&b->q32, link_off * sizeof(float4)), "cudaMalloc(links)");
   }
@@ -750,12 +746,11 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
   // the trials advance the batch: save links, streams, counters, cursors and
   // series, restore them afterwards
   struct Saved {
-    void *l0 = nullptr, *l1 = nullptr, *rng = nullptr, *acc = nullptr, *draw = nullptr, *cur = nullptr,
+    void *l0 = nullptr, *rng = nullptr, *acc = nullptr, *draw = nullptr, *cur = nullptr,
          *ser = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ~Saved() {
       cudaFree(l0);
-      cudaFree(l1);
       cudaFree(rng);
       cudaFree(acc);
       cudaFree(draw);
@@ -767,15 +762,13 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
   } sv;
   long long links = 0;
   for (int r = 0; r < b->n; r++) links += link_bytes_of(b, r);
-  const size_t lb = fp64(b) ? (size_t)links / 2 : (size_t)links;  // per store (FP64: lo and hi)
+  const size_t lb = (size_t)links;
   const size_t rngb = (size_t)(b->sites / 2) * 6 * sizeof(uint32_t);
   const size_t serb = (size_t)b->cap * b->n * sizeof(double2);
-  void* L0 = fp64(b) ? (void*)b->lo : (void*)b->q32;
+  void* L0 = fp64(b) ? (void*)b->q64 : (void*)b->q32;
   BCUDA(b, cudaMalloc(&sv.l0, lb));
   BCUDA(b, cudaMemcpyAsync(sv.l0, L0, lb, cudaMemcpyDeviceToDevice, b->stream));
   if (fp64(b)) {
-    BCUDA(b, cudaMalloc(&sv.l1, lb));
-    BCUDA(b, cudaMemcpyAsync(sv.l1, b->hi, lb, cudaMemcpyDeviceToDevice, b->stream));
     BCUDA(b, cudaMalloc(&sv.rng, rngb));
     BCUDA(b, cudaMemcpyAsync(sv.rng, b->rng, rngb, cudaMemcpyDeviceToDevice, b->stream));
   }
@@ -844,7 +837,6 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
   // restore the batch as it was
   cudaMemcpyAsync(L0, sv.l0, lb, cudaMemcpyDeviceToDevice, b->stream);
   if (fp64(b)) {
-    cudaMemcpyAsync(b->hi, sv.l1, lb, cudaMemcpyDeviceToDevice, b->stream);
     cudaMemcpyAsync(b->rng, sv.rng, rngb, cudaMemcpyDeviceToDevice, b->stream);
   }
   if (sv.acc) cudaMemcpyAsync(b->accept, sv.acc, (size_t)b->sites * sizeof(int), cudaMemcpyDeviceToDevice, b->stream);
@@ -913,19 +905,13 @@ int qcd_batch_store_config(qcd_batch* b, int replica, double* aos_host) {
   const size_t vh = (size_t)R.g.vh;
   // SoA planes -> the reference's AoS layout, on the host
   if (fp64(b)) {
-    std::vector<double2> lo(6 * vh), hi(6 * vh);
-    BCUDA(b, cudaMemcpy(lo.data(), b->lo + R.link_off, 6 * vh * sizeof(double2), cudaMemcpyDeviceToHost));
-    BCUDA(b, cudaMemcpy(hi.data(), b->hi + R.link_off, 6 * vh * sizeof(double2), cudaMemcpyDeviceToHost));
+    std::vector<double> q(24 * vh);
+    BCUDA(b, cudaMemcpy(q.data(), b->q64 + 4 * R.link_off, 24 * vh * sizeof(double), cudaMemcpyDeviceToHost));
     for (int p = 0; p < 2; p++)
       for (size_t id = 0; id < vh; id++)
-        for (int d = 0; d < 3; d++) {
-          const size_t i = (size_t)(d * 2 + p) * vh + id;
-          double* s = aos_host + ((size_t)p * vh + id) * 12 + d * 4;
-          s[0] = lo[i].x;
-          s[1] = lo[i].y;
-          s[2] = hi[i].x;
-          s[3] = hi[i].y;
-        }
+        for (int d = 0; d < 3; d++)
+          memcpy(aos_host + ((size_t)p * vh + id) * 12 + d * 4, &q[((size_t)(d * 2 + p) * vh + id) * 4],
+                 4 * sizeof(double));
   } else {
     std::vector<float4> q(6 * vh);
     BCUDA(b, cudaMemcpy(q.data(), b->q32 + R.link_off, 6 * vh * sizeof(float4), cudaMemcpyDeviceToHost));

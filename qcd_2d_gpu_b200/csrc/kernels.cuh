@@ -13,12 +13,12 @@
 namespace qcd {
 
 // ------------------------------------------------------------ one phase --
-// Launch grid tile_grid(g), kTileThreads threads.  FP64 CTAs per SM, measured:
-// over-relaxation nine (56 registers; 128^3 pass 211 us, 216 at eight, 239 at the
-// compiler's choice), heat-bath and Metropolis seven (72; heat-bath 64^3 40.6 us,
-// 42.1 at nine, 45.8 at six; Metropolis 64^3 65.6 us, 72 at six).
+// Launch grid tile_grid(g), kTileThreads threads.  FP64 CTAs per SM, measured: seven (72
+// registers) for every kind; over-relaxation passes 48x64x80 22.9 us and 128^3 197 us
+// (24.9 and 201 at nine), heat-bath 64^3 40.1 and 128^3 283 us (40.6 and 288 at nine, 45.0
+// and 294 at six), Metropolis 64^3 63.2 us (64.5 at eight, 69.9 at six).
 template <int MU, int PAR, int BC, int KIND>
-__global__ void __launch_bounds__(kTileThreads, KIND == KIND_OR ? 9 : 7) phase64(Links64 L, RngStore R, Geo g, PhaseArgs a) {
+__global__ void __launch_bounds__(kTileThreads, 7) phase64(Links64 L, RngStore R, Geo g, PhaseArgs a) {
   Nbr n;
   if (!tile_nbr<PAR>(g, n)) return;
   if (KIND != KIND_OR) count_draws(a);

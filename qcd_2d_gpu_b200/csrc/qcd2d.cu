@@ -28,8 +28,7 @@ struct qcd_lattice {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   // link store
-  double2* lo = nullptr;
-  double2* hi = nullptr;
+  double* q64 = nullptr;
   float4* q32 = nullptr;     // FP32 store holding the current links
   float4* q32alt = nullptr;  // second FP32 store: the fused-pair schedule writes each pass's new links here
   size_t link_bytes = 0;
@@ -112,7 +111,7 @@ int fail(qcd_lattice* h, int code, const char* fmt, ...) {
 
 inline unsigned int nblocks(long long n) { return (unsigned int)((n + kBlock - 1) / kBlock); }
 
-Links64 links64(const qcd_lattice* h) { return Links64{h->lo, h->hi, h->g.vh}; }
+Links64 links64(const qcd_lattice* h) { return Links64{h->q64, h->g.vh}; }
 Links32 links32(const qcd_lattice* h) { return Links32{h->q32, h->g.vh}; }
 Pair32 pair32(const qcd_lattice* h) { return Pair32{h->q32, h->g.vh / 2}; }
 bool pairable(const qcd_lattice* h) { return h->p.precision == QCD_PREC_FP32 && h->g.lt % 4 == 0; }
@@ -449,7 +448,7 @@ int launch_wave(qcd_lattice* h, const PassSpec* ps, int np, int stall_test = 0,
   const unsigned int grid = (unsigned int)h->wave_grid;
   RngStore R{h->rng, h->g.vh};
   if (h->p.precision == QCD_PREC_FP64) {
-    Links64T<true> L{h->lo, h->hi, h->g.vh};
+    Links64T<true> L{h->q64, h->g.vh};
     if (sk == KIND_HB) {
       if (bc == 0) wave<Links64T<true>, 0, KIND_HB><<<grid, kBlock, 0, h->stream>>>(L, R, h->g, a, S, c);
       else if (bc == 1) wave<Links64T<true>, 1, KIND_HB><<<grid, kBlock, 0, h->stream>>>(L, R, h->g, a, S, c);
@@ -722,8 +721,7 @@ int ensure_rng(qcd_lattice* h) {
 }
 
 void release(qcd_lattice* h) {
-  cudaFree(h->lo);
-  cudaFree(h->hi);
+  cudaFree(h->q64);
   cudaFree(h->q32);
   cudaFree(h->q32alt);
   cudaFree(h->rng);
@@ -815,9 +813,8 @@ int qcd_create(const qcd_params* p, qcd_lattice** out) {
   step(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking), "cudaStreamCreate");
   h->stream = h->own_stream;
   if (p->precision == QCD_PREC_FP64) {
-    h->link_bytes = 6 * vh * sizeof(double2) * 2;
-    if (rc == QCD_OK) step(cudaMalloc(&h->lo, 6 * vh * sizeof(double2)), "cudaMalloc(links)");
-    if (rc == QCD_OK) step(cudaMalloc(&h->hi, 6 * vh * sizeof(double2)), "cudaMalloc(links)");
+    h->link_bytes = 6 * vh * 4 * sizeof(double);
+    if (rc == QCD_OK) step(cudaMalloc(&h->q64, h->link_bytes), "cudaMalloc(links)");
   } else {
     h->link_bytes = 6 * vh * sizeof(float4);
     if (rc == QCD_OK) step(cudaMalloc(&h->q32, 6 * vh * sizeof(float4)), "cudaMalloc(links)");
@@ -1144,27 +1141,24 @@ int qcd_autotune(qcd_lattice* h, int sweeps_per_trial, qcd_tuning* chosen) {
   // the backups are freed on every way out of this function (a failed
   // allocation or copy returns early)
   struct Backups {
-    void *links = nullptr, *links2 = nullptr, *rng = nullptr, *acc = nullptr;
+    void *links = nullptr, *rng = nullptr, *acc = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ~Backups() {
       cudaFree(links);
-      cudaFree(links2);
       cudaFree(rng);
       cudaFree(acc);
       if (e0) cudaEventDestroy(e0);
       if (e1) cudaEventDestroy(e1);
     }
   } bk;
-  void *&links_save = bk.links, *&links2_save = bk.links2, *&rng_save = bk.rng, *&acc_save = bk.acc;
-  const size_t lb = h->p.precision == QCD_PREC_FP64 ? h->link_bytes / 2 : h->link_bytes;
+  void *&links_save = bk.links, *&rng_save = bk.rng, *&acc_save = bk.acc;
+  const size_t lb = h->link_bytes;
   // (the fused pairs swap the FP32 stores: the restore goes to whichever is current then)
-  void* lp = h->p.precision == QCD_PREC_FP64 ? (void*)h->lo : (void*)h->q32;
+  void* lp = h->p.precision == QCD_PREC_FP64 ? (void*)h->q64 : (void*)h->q32;
   CUDA_OR_FAIL(h, cudaMalloc(&links_save, lb));
-  if (h->p.precision == QCD_PREC_FP64) CUDA_OR_FAIL(h, cudaMalloc(&links2_save, lb));
   if (h->rng) CUDA_OR_FAIL(h, cudaMalloc(&rng_save, rng_bytes));
   if (h->accept) CUDA_OR_FAIL(h, cudaMalloc(&acc_save, (size_t)h->V * sizeof(int)));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(links_save, lp, lb, cudaMemcpyDeviceToDevice, h->stream));
-  if (links2_save) CUDA_OR_FAIL(h, cudaMemcpyAsync(links2_save, h->hi, lb, cudaMemcpyDeviceToDevice, h->stream));
   if (rng_save) CUDA_OR_FAIL(h, cudaMemcpyAsync(rng_save, h->rng, rng_bytes, cudaMemcpyDeviceToDevice, h->stream));
   if (acc_save)
     CUDA_OR_FAIL(h, cudaMemcpyAsync(acc_save, h->accept, (size_t)h->V * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
@@ -1192,9 +1186,8 @@ int qcd_autotune(qcd_lattice* h, int sweeps_per_trial, qcd_tuning* chosen) {
     if (rc == QCD_OK && cand[i].ms_per_sweep < cand[best].ms_per_sweep) best = (int)i;
   }
   // restore the lattice as it was
-  lp = h->p.precision == QCD_PREC_FP64 ? (void*)h->lo : (void*)h->q32;
+  lp = h->p.precision == QCD_PREC_FP64 ? (void*)h->q64 : (void*)h->q32;
   cudaMemcpyAsync(lp, links_save, lb, cudaMemcpyDeviceToDevice, h->stream);
-  if (links2_save) cudaMemcpyAsync(h->hi, links2_save, lb, cudaMemcpyDeviceToDevice, h->stream);
   if (rng_save) cudaMemcpyAsync(h->rng, rng_save, rng_bytes, cudaMemcpyDeviceToDevice, h->stream);
   if (acc_save) cudaMemcpyAsync(h->accept, acc_save, (size_t)h->V * sizeof(int), cudaMemcpyDeviceToDevice, h->stream);
   cudaStreamSynchronize(h->stream);
@@ -1389,7 +1382,7 @@ int qcd_get_params(const qcd_lattice* h, qcd_params* out) {
 
 int qcd_link_store(const qcd_lattice* h, void** dev_ptr, size_t* bytes) {
   if (!h) return QCD_ERR_INVALID;
-  if (dev_ptr) *dev_ptr = h->p.precision == QCD_PREC_FP64 ? (void*)h->lo : (void*)h->q32;
+  if (dev_ptr) *dev_ptr = h->p.precision == QCD_PREC_FP64 ? (void*)h->q64 : (void*)h->q32;
   if (bytes) *bytes = h->link_bytes;
   return QCD_OK;
 }
@@ -1427,8 +1420,13 @@ namespace qcd {
 struct LinksAoS {
   const double* phi;  // V*12 doubles: site (p*Vh + id), link d, component c
   int vh;
+  // phi is 32-byte aligned, and with it every link: one 256-bit load per link (the
+  // 96-byte stride of the sites makes the number of load instructions the bound:
+  // 160x144x176 106-114 -> 91-100 us)
+  bool wide;
   __device__ __forceinline__ Quat<double> ld(int d, int p, int id) const {
     const double* s = phi + ((size_t)p * vh + id) * 12 + d * 4;
+    if (wide) return ld_link_nc(s);
     double2 a = __ldg(reinterpret_cast<const double2*>(s));
     double2 b = __ldg(reinterpret_cast<const double2*>(s + 2));
     return Quat<double>{a.x, a.y, b.x, b.y};
@@ -1497,7 +1495,7 @@ extern "C" int qcd_measure_aos_noalloc(const double* phi_dev, int lt, int lx, in
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), s);
   if (e == cudaSuccess) {
     Geo g = make_geo(lt, lx, ly);
-    LinksAoS L{phi_dev, (int)vh};
+    LinksAoS L{phi_dev, (int)vh, ((uintptr_t)phi_dev & 31) == 0};
     const unsigned int grid = measure_blocks(vh, kMeasurePerSM64);  // the same grid, so the same sums, as qcd_measure
     if (boundary == QCD_BC_PMC)
       measure<LinksAoS, 1, kMeasurePerSM64><<<grid, kBlock, 0, s>>>(L, g, partials, counter, out_dev, nullptr);
