@@ -89,7 +89,6 @@ __global__ void __launch_bounds__(kBlock, FP64 ? 4 : 5) batch_phase(BatchView B,
   PhaseArgs pa{R.beta, a.eps, a.upd, a.err, a.accept ? a.accept + R.site_off : nullptr, a.renorm,
                R.seed, a.phase_ptr, a.phase_off, (unsigned int)R.stream_off, philox_keys(R.seed), a.count_out,
                a.count_add};
-  if (KIND != KIND_OR) count_draws(pa);
   RngStore RS{B.rng + R.rng_off, R.g.vh};
   if (FP64) {
     Links64 L{B.q64 + 4 * R.link_off, R.g.vh};
@@ -106,6 +105,7 @@ __global__ void __launch_bounds__(kBlock, FP64 ? 4 : 5) batch_phase(BatchView B,
       default: site32<MU, PAR, BC_PMC, KIND, false>(L, RS, R.g, pa, n, a.renorm); break;
     }
   }
+  if (KIND != KIND_OR) count_draws(pa);
 }
 
 // curand_init(seed_r, stream_off_r + id, 0) per site of every replica (one

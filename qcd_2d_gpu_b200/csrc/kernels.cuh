@@ -21,8 +21,8 @@ template <int MU, int PAR, int BC, int KIND>
 __global__ void __launch_bounds__(kTileThreads, 7) phase64(Links64 L, RngStore R, Geo g, PhaseArgs a) {
   Nbr n;
   if (!tile_nbr<PAR>(g, n)) return;
-  if (KIND != KIND_OR) count_draws(a);
   site64<MU, PAR, BC, KIND, false>(L, R, g, a, n);
+  if (KIND != KIND_OR) count_draws(a);
 }
 
 // FP32 planes: eight CTAs per SM, which leaves registers to ask for several links at
@@ -32,8 +32,8 @@ template <int MU, int PAR, int BC, int KIND>
 __global__ void __launch_bounds__(kTileThreads, 8) phase32(Links32 L, RngStore R, Geo g, PhaseArgs a) {
   Nbr n;
   if (!tile_nbr<PAR>(g, n)) return;
-  if (KIND != KIND_OR) count_draws(a);
   site32<MU, PAR, BC, KIND, false>(L, R, g, a, n, a.renorm);
+  if (KIND != KIND_OR) count_draws(a);
 }
 
 // ------------------------------------------------------------ RNG setup --

@@ -191,18 +191,24 @@ __device__ __forceinline__ bool at_ytop(const Geo& g, const Nbr& n) {
 
 __host__ __device__ __forceinline__ size_t plane_of(int dir, int parity) { return (size_t)(dir * 2 + parity); }
 
-// Load/store policy: CG = false uses the read-only path (__ldg) for neighbour
-// links, which is safe inside one phase launch because no link a phase reads
-// is written in that launch.  CG = true (the wavefront kernel) reads and
-// writes at L2 (.cg): there, other CTAs of the same launch rewrite links, and
-// a line left in this SM's L1 by an earlier task could be stale.  The link a
-// thread rewrites is read at L2 in either case: its sector may hold a link that
-// another SM rewrites in the same launch, and the next launch's CTAs may already
-// be set up on this SM.
-template <class T, bool CG>
-__device__ __forceinline__ T ld_nb(const T* p) {
-  if (CG) return __ldcg(p);
-  return __ldg(p);
+// Load/store policy: CG = false reads neighbour links by ordinary loads, which may
+// hit in L1: no link that a phase reads so is written in that launch.  Not by the
+// non-coherent path (ld.global.nc, __ldg): that one asks for data that nothing writes
+// while the kernel lives, and a chained launch is alive while its predecessor still
+// writes.  Ordinary loads after chain_wait see the predecessor's writes by the memory
+// model; both go through L1, and the passes take the same time to 1%.
+// CG = true (the wavefront kernel) reads and writes at L2 (.cg): there, other CTAs of
+// the same launch rewrite links, and a line left in this SM's L1 by an earlier task
+// could be stale.  The link a thread rewrites is read at L2 in either case: its sector
+// may hold a link that another SM rewrites in the same launch, and the next launch's
+// CTAs may already be set up on this SM.
+//
+// ld_float4, ld_link and ld_pair are not volatile, so they can be scheduled among other
+// loads: nothing that a kernel reads through them is written by that kernel.
+__device__ __forceinline__ float4 ld_float4(const float4* p) {
+  float4 v;
+  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
 }
 template <class T, bool CG>
 __device__ __forceinline__ void st_rw(T* p, const T& v) {
@@ -217,9 +223,9 @@ __device__ __forceinline__ void st_rw(T* p, const T& v) {
 // the load instructions and addresses of two double2 planes (passes: heat-bath 128^3
 // 285 -> 275 us, 256^3 2.57 -> 2.49 ms, over-relaxation 128^3 210 -> 201 us; measurement
 // 256^3 306 -> 290 us).
-__device__ __forceinline__ Quat<double> ld_link_nc(const double* p) {
+__device__ __forceinline__ Quat<double> ld_link(const double* p) {
   Quat<double> u;
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(u.w), "=d"(u.x), "=d"(u.y), "=d"(u.z) : "l"(p));
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(u.w), "=d"(u.x), "=d"(u.y), "=d"(u.z) : "l"(p));
   return u;
 }
 __device__ __forceinline__ Quat<double> ld_link_cg(const double* p) {
@@ -238,7 +244,7 @@ struct Links64T {
     return q + (plane_of(dir, parity) * vh + id) * 4;
   }
   __device__ __forceinline__ Quat<double> ld(int dir, int parity, int id) const {
-    return CG ? ld_link_cg(at(dir, parity, id)) : ld_link_nc(at(dir, parity, id));
+    return CG ? ld_link_cg(at(dir, parity, id)) : ld_link(at(dir, parity, id));
   }
   // the link this thread rewrites
   __device__ __forceinline__ Quat<double> ld_own(int dir, int parity, int id) const {
@@ -263,7 +269,8 @@ struct Links32T {
   float4* q;
   int vh;
   __device__ __forceinline__ Quat<float> ld(int dir, int parity, int id) const {
-    float4 a = ld_nb<float4, CG>(q + plane_of(dir, parity) * vh + id);
+    const float4* p = q + plane_of(dir, parity) * vh + id;
+    const float4 a = CG ? __ldcg(p) : ld_float4(p);
     return Quat<float>{a.x, a.y, a.z, a.w};
   }
   __device__ __forceinline__ Quat<float> ld_own(int dir, int parity, int id) const {

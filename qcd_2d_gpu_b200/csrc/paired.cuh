@@ -95,14 +95,14 @@ __device__ __forceinline__ float2 p2_retr_bd(const Q2& a, const Q2& b) {
 // One pair record in one 32-B access (sm_100 global loads and stores of
 // eight 32-bit words; the record is 32-B aligned): half the load
 // instructions and L1 wavefronts of two float4 accesses.
-__device__ __forceinline__ Q2 ld_pair_nc(const float4* p) {
+__device__ __forceinline__ Q2 ld_pair(const float4* p) {
   float a0, a1, a2, a3, b0, b1, b2, b3;
-  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+  asm("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=f"(a0), "=f"(a1), "=f"(a2), "=f"(a3), "=f"(b0), "=f"(b1), "=f"(b2), "=f"(b3)
       : "l"(p));
   return Q2{f2(a0, a1), f2(a2, a3), f2(b0, b1), f2(b2, b3)};
 }
-__device__ __forceinline__ Q2 ld_pair(const float4* p) {
+__device__ __forceinline__ Q2 ld_pair_cg(const float4* p) {
   float a0, a1, a2, a3, b0, b1, b2, b3;
   asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=f"(a0), "=f"(a1), "=f"(a2), "=f"(a3), "=f"(b0), "=f"(b1), "=f"(b2), "=f"(b3)
@@ -124,9 +124,9 @@ struct Pair32 {
     return q + ((size_t)plane_of(dir, par) * vhp + j) * 2;
   }
   // a neighbour pair (not written by the launch that reads it)
-  __device__ __forceinline__ Q2 ld(int dir, int par, int j) const { return ld_pair_nc(at(dir, par, j)); }
+  __device__ __forceinline__ Q2 ld(int dir, int par, int j) const { return ld_pair(at(dir, par, j)); }
   // the pair a thread rewrites
-  __device__ __forceinline__ Q2 ld_own(int dir, int par, int j) const { return ld_pair(at(dir, par, j)); }
+  __device__ __forceinline__ Q2 ld_own(int dir, int par, int j) const { return ld_pair_cg(at(dir, par, j)); }
   __device__ __forceinline__ void st(int dir, int par, int j, const Q2& u) const { st_pair(at(dir, par, j), u); }
   // one site, by its sublattice index (the one-off kernels: starts, layout changes)
   __device__ __forceinline__ Quat<float> ld_site(int dir, int par, int id) const {
@@ -310,12 +310,13 @@ template <int MU, int PAR, int BC, int KIND>
 __global__ void __launch_bounds__(kTileThreads, 8) phase32p(Pair32 P, Geo gh, PhaseArgs a) {
   Nbr n;
   if (!tile_nbr<PAR>(gh, n)) return;
+  if (!(BC == BC_PCC && MU != DIR_Y && at_y0(gh, n))) {
+    const Q2 A = staple_sum2<MU, BC>(P, gh, n, PAR, n.t == gh.lt - 1, n.t == 0);
+    const Q2 U = pair_new<KIND>(P, A, a, MU, PAR, n.id, a.renorm);
+    chain_ready();
+    P.st(MU, PAR, n.id, U);
+  }
   if (KIND != KIND_OR) count_draws(a);
-  if (BC == BC_PCC && MU != DIR_Y && at_y0(gh, n)) return;
-  const Q2 A = staple_sum2<MU, BC>(P, gh, n, PAR, n.t == gh.lt - 1, n.t == 0);
-  const Q2 U = pair_new<KIND>(P, A, a, MU, PAR, n.id, a.renorm);
-  chain_ready();
-  P.st(MU, PAR, n.id, U);
 }
 
 // ------------------------------------------------------- measurement ----

@@ -1426,7 +1426,7 @@ struct LinksAoS {
   bool wide;
   __device__ __forceinline__ Quat<double> ld(int d, int p, int id) const {
     const double* s = phi + ((size_t)p * vh + id) * 12 + d * 4;
-    if (wide) return ld_link_nc(s);
+    if (wide) return ld_link(s);
     double2 a = __ldg(reinterpret_cast<const double2*>(s));
     double2 b = __ldg(reinterpret_cast<const double2*>(s + 2));
     return Quat<double>{a.x, a.y, b.x, b.y};
