@@ -94,14 +94,14 @@ int fail(qcd_lattice* h, int code, const char* fmt, ...) {
   return code;
 }
 
+// (the runtime's record of the error is cleared: a later call must not report it again)
 #define CUDA_OR_FAIL(h, call)                                                                 \
   do {                                                                                        \
     cudaError_t e_ = (call);                                                                  \
     if (e_ != cudaSuccess) {                                                                  \
-      if (e_ == cudaErrorMemoryAllocation) {                                                  \
-        cudaGetLastError();                                                                   \
+      cudaGetLastError();                                                                     \
+      if (e_ == cudaErrorMemoryAllocation)                                                    \
         return fail(h, QCD_ERR_NOMEM, "%s: %s", #call, cudaGetErrorString(e_));               \
-      }                                                                                       \
       return fail(h, QCD_ERR_CUDA, "%s (%s:%d): %s", #call, __FILE__, __LINE__,               \
                   cudaGetErrorString(e_));                                                    \
     }                                                                                         \
