@@ -18,6 +18,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <mutex>
 #include <new>
 #include <utility>
 #include <vector>
@@ -306,8 +307,9 @@ struct qcd_batch {
   double2* series = nullptr;
   int cap = 0;
   // pinned staging of what the host reads back: kBatchStage pairs of a series, then
-  // the device error word
+  // the device error word; threads that read series take turns at it
   double2* stage = nullptr;
+  std::mutex stage_turn;
   long long sweeps_done = 0;
   std::vector<BatchGroup> groups;
   long long group_bytes = 0;  // target link bytes per group (0: one group)
@@ -859,8 +861,8 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
   return QCD_OK;
 }
 
-int qcd_batch_synchronize(qcd_batch* b) {
-  if (!b) return QCD_ERR_INVALID;
+// waits for the batch's stream and reads the error word (the caller has stage_turn)
+static int wait_and_check(qcd_batch* b) {
   int e = 0;
   BCUDA(b, cudaMemcpyAsync(b->stage + kBatchStage, b->err, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   BCUDA(b, cudaStreamSynchronize(b->stream));
@@ -868,6 +870,12 @@ int qcd_batch_synchronize(qcd_batch* b) {
   if (e & DEVERR_HB_LOOP)
     return bfail(b, QCD_ERR_NONUNITARY, "heat-bath rejection loop exceeded %d tries", QCD_HB_MAX_TRIES);
   return QCD_OK;
+}
+
+int qcd_batch_synchronize(qcd_batch* b) {
+  if (!b) return QCD_ERR_INVALID;
+  std::lock_guard<std::mutex> turn(b->stage_turn);
+  return wait_and_check(b);
 }
 
 int qcd_batch_measured(qcd_batch* b) {
@@ -882,12 +890,13 @@ int qcd_batch_series(qcd_batch* b, int replica, double* energy, double* plaquett
   if (!b || replica < 0 || replica >= b->n || n < 0 || n > b->cap) return QCD_ERR_INVALID;
   // the first pairs and the error word come with one wait (a read per replica is what
   // a program does after a run: 96 of them 2.8 ms with a wait for each and pageable copies)
+  std::lock_guard<std::mutex> turn(b->stage_turn);
   for (int i0 = 0; i0 == 0 || i0 < n; i0 += kBatchStage) {
     const int m = n - i0 < kBatchStage ? n - i0 : kBatchStage;
     if (m > 0)
       BCUDA(b, cudaMemcpyAsync(b->stage, b->series + (size_t)replica * b->cap + i0, m * sizeof(double2),
                                cudaMemcpyDeviceToHost, b->stream));
-    int rc = qcd_batch_synchronize(b);
+    int rc = wait_and_check(b);
     if (rc) return rc;
     for (int i = 0; i < m; i++) {
       if (energy) energy[i0 + i] = b->stage[i].x;
