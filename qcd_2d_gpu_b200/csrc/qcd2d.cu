@@ -970,13 +970,15 @@ int qcd_sweep(qcd_lattice* h, int n) {
     // re-projected at its last update (no extra read of the store); FP64
     // keeps the reference's separate normalize after the sweep
     const bool fused = renorm && h->p.precision == QCD_PREC_FP32;
-    if (np + 1 + h->p.n_or > 64) {
-      int rc = run_passes(h, buf, np);
-      if (rc) return rc;
-      np = 0;
+    // (a sweep may have more over-relaxation passes than the list holds)
+    for (int r = -1; r < h->p.n_or; r++) {
+      if (np == 64) {
+        int rc = run_passes(h, buf, np);
+        if (rc) return rc;
+        np = 0;
+      }
+      buf[np++] = PassSpec{r < 0 ? kind : KIND_OR, fused && r == h->p.n_or - 1};
     }
-    buf[np++] = PassSpec{kind, fused && h->p.n_or == 0};
-    for (int r = 0; r < h->p.n_or; r++) buf[np++] = PassSpec{KIND_OR, fused && r == h->p.n_or - 1};
     h->sweeps_done++;
     if (renorm && !fused) {
       int rc = run_passes(h, buf, np);
