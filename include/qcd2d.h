@@ -176,6 +176,13 @@ enum qcd_schedule { QCD_SCHED_AUTO = 0, QCD_SCHED_PHASES = 1, QCD_SCHED_WAVEFRON
 int qcd_set_schedule(qcd_lattice* h, int mode);
 /* the schedule qcd_sweep will use (PHASES, WAVEFRONT or PAIRS) */
 int qcd_get_schedule(const qcd_lattice* h);
+/* PHASES on a small lattice: on = 1 (the default) lets its passes run in one
+   cluster, on = 0 keeps a launch per phase.  Links, draws and counters are the
+   same bit for bit. */
+int qcd_set_cluster(qcd_lattice* h, int on);
+/* 1 if the next pass runs in a cluster, 0 if not (also asks the device, once per
+   store layout, whether it can hold one) */
+int qcd_get_cluster(qcd_lattice* h);
 /* FP32 store layout.  An FP32 lattice with Lt % 4 == 0 keeps its links in
    site pairs under the per-phase schedule: site id (t < Lt/2) and site
    id + V/4 (t + Lt/2) of a link class share one 32-B record (w0 w1 x0 x1)

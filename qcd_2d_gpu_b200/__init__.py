@@ -156,6 +156,8 @@ _SIGS = {
     "qcd_get_schedule": (_I, [_P]),
     "qcd_set_pair_layout": (_I, [_P, _I]),
     "qcd_get_pair_layout": (_I, [_P]),
+    "qcd_set_cluster": (_I, [_P, _I]),
+    "qcd_get_cluster": (_I, [_P]),
     "qcd_wave_plan": (_I, [_P, _P, _I, _P, _P, _P]),
     "qcd_wave_selftest_timeout": (_I, [_P]),
     "qcd_set_wave_tuning": (_I, [_P, _I, _I, _I]),
@@ -300,6 +302,15 @@ class Lattice:
 
     def pair_layout(self) -> bool:
         return self._lib.qcd_get_pair_layout(self._h) == 1
+
+    def set_cluster(self, on: bool) -> None:
+        """Per-phase schedule: let a small lattice's passes run in one cluster (True, the
+        default) or keep a launch per phase; the results are the same."""
+        self._check(self._lib.qcd_set_cluster(self._h, int(bool(on))), "set_cluster")
+
+    def cluster(self) -> bool:
+        """Whether the next pass runs in a cluster."""
+        return self._lib.qcd_get_cluster(self._h) == 1
 
     def set_wave_tuning(self, chunk_sites: int = 0, passes_per_launch: int = 0, fronts: int = 0) -> None:
         self._check(self._lib.qcd_set_wave_tuning(self._h, chunk_sites, passes_per_launch, fronts),

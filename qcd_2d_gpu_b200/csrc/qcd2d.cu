@@ -73,6 +73,7 @@ struct qcd_lattice {
   int wave_tasks_chunk[5] = {0, 0, 0, 0, 0};
   int wave_tasks_fronts[5] = {0, 0, 0, 0, 0};
   int sms = 0;       // multiprocessors of the device (fused pairs)
+  bool resident_ok = true;  // qcd_set_cluster: the cluster route allowed
   int resident_can[2] = {-1, -1};  // small lattices: one cluster can hold the passes (planes, pairs; -1: not asked)
   // fused pairs: the two FP32 stores and their tensor maps (pair_buf[0] is
   // the store allocated at create; q32 / q32alt point at one each)
@@ -534,6 +535,7 @@ cudaError_t resident_call(const qcd_lattice* h, const ResidentProgram& p, bool p
 // Whether the per-phase schedule runs this lattice's passes in one cluster (asked
 // of the device once per store layout).
 bool use_resident(qcd_lattice* h) {
+  if (!h->resident_ok) return false;
   const bool planes32 = h->p.precision == QCD_PREC_FP32 && !h->paired;
   const int most = h->p.algo == QCD_ALGO_METROPOLIS && !planes32 ? kResidentItemsMetro : kResidentItems;
   if ((h->paired ? h->gh.vh : h->g.vh) > most) return false;
@@ -1060,6 +1062,17 @@ int qcd_get_pair_layout(const qcd_lattice* h) {
 int qcd_get_schedule(const qcd_lattice* h) {
   if (!h) return QCD_ERR_INVALID;
   return use_pairs(h) ? QCD_SCHED_PAIRS : use_wave(h) ? QCD_SCHED_WAVEFRONT : QCD_SCHED_PHASES;
+}
+
+int qcd_set_cluster(qcd_lattice* h, int on) {
+  if (!h || on < 0 || on > 1) return QCD_ERR_INVALID;
+  h->resident_ok = on != 0;
+  return QCD_OK;
+}
+
+int qcd_get_cluster(qcd_lattice* h) {
+  if (!h) return QCD_ERR_INVALID;
+  return !use_pairs(h) && !use_wave(h) && use_resident(h) ? 1 : 0;
 }
 
 int qcd_set_pair_tuning(qcd_lattice* h, int slices_per_cta) {
