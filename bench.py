@@ -585,10 +585,9 @@ def main():
         except Exception:
             pass
     if roofline["traffic"]:
-        # the DRAM bytes a launch really moves (ncu) over its live time: how close
-        # the kernel runs to HBM for the traffic of its per-phase design
-        roofline["traffic_gbs"] = roofline["traffic"] / (or_launch_ms * 1e-3) / 1e9
-        roofline["traffic_frac"] = roofline["traffic_gbs"] / hbm
+        # no rate is formed from these bytes and the live time: in a run the odd phases
+        # start on links that the even ones left in L2, and fewer bytes move
+        roofline["traffic_of"] = "DRAM bytes of one launch alone, caches cold (ncu)"
 
     # ---- the reference arm's workload on our kernels ------------------------
     # (heat-bath only, a measurement every N_COR sweeps): the like-for-like
