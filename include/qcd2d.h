@@ -392,9 +392,9 @@ int qcd_rng_tape(unsigned long long seed, long long first, int n_streams, int n_
  * a fixed array inside the library, present on every GPU that loads it until
  * the process exits.
  *
- * Limits: the scratch holds QCD_NOALLOC_MAX_BLOCKS partial sums (64 KB), which
- * is the most CTAs any measurement launches, whatever the lattice size: the
- * threads of a CTA stride over the sites.  The lattice itself is bounded only
+ * Limits: the scratch holds QCD_NOALLOC_MAX_BLOCKS partial sums (64 KB), far
+ * more than the CTAs a measurement launches (296 at most, whatever the lattice
+ * size: the threads of a CTA stride over the sites).  The lattice itself is bounded only
  * by the 32-bit site indices, V/2 <= QCD_NOALLOC_MAX_HALF_SITES (the same bound
  * as qcd_create; 384^3 and larger fit); beyond it the call returns
  * QCD_ERR_UNSUPPORTED (and says so on stderr) without touching the device.

@@ -176,9 +176,9 @@ __global__ void __launch_bounds__(kBlock) batch_normalize(BatchView B) {
 // CTA adds their partials in the same order, so every replica's numbers are
 // those of the same lattice measured alone, bit for bit.
 template <bool FP64>
-__global__ void __launch_bounds__(kBlock, FP64 ? kMeasurePerSM64 : kMeasurePerSM32) batch_measure(BatchView B, double2* partials, unsigned int* rep_count,
-                                                        unsigned int* all_count, int* cursor, double2* series,
-                                                        int cap) {
+__global__ void __launch_bounds__(kBlock, FP64 ? kMeasurePerSM64 : kMeasurePerSM32)
+    batch_measure(BatchView B, double2* partials, unsigned int* rep_count, unsigned int* all_count, int* cursor,
+                  double2* series, int cap) {
   const int mcta = (int)blockIdx.x + B.mcta0;  // CTA in the batch's measurement table
   const int r = __ldg(B.mcta_rep + mcta);
   const Replica& R = B.rep[r];
@@ -420,7 +420,8 @@ int batch_sweep(qcd_batch* b, int gi, bool renorm) {
   const int kind = b->common.algo == QCD_ALGO_HEATBATH ? KIND_HB : KIND_METRO;
   const bool fused = renorm && !fp64(b);
   int rc = batch_pass(b, gi, kind, fused && b->common.n_or == 0);
-  for (int r = 0; rc == QCD_OK && r < b->common.n_or; r++) rc = batch_pass(b, gi, KIND_OR, fused && r == b->common.n_or - 1);
+  for (int r = 0; rc == QCD_OK && r < b->common.n_or; r++)
+    rc = batch_pass(b, gi, KIND_OR, fused && r == b->common.n_or - 1);
   if (rc) return rc;
   if (renorm && !fused) {
     const BatchGroup& g = b->groups[gi];
@@ -435,8 +436,9 @@ int batch_sweep(qcd_batch* b, int gi, bool renorm) {
 
 int batch_measure_launch(qcd_batch* b, int gi) {
   const BatchGroup& g = b->groups[gi];
-  BCUDA(b, launch_chained(fp64(b) ? batch_measure<true> : batch_measure<false>, g.mctas, kBlock, b->stream, view(b, g),
-                          b->partials, b->rep_count, b->all_count + gi, b->cursor + gi, b->series, b->cap));
+  BCUDA(b, launch_chained(fp64(b) ? batch_measure<true> : batch_measure<false>, g.mctas, kBlock, b->stream,
+                          view(b, g), b->partials, b->rep_count, b->all_count + gi, b->cursor + gi, b->series,
+                          b->cap));
   return QCD_OK;
 }
 
@@ -480,7 +482,8 @@ int qcd_batch_create(const qcd_replica* r, int n, const qcd_params* common, qcd_
   if (common->algo != QCD_ALGO_HEATBATH && common->algo != QCD_ALGO_METROPOLIS) return QCD_ERR_INVALID;
   if (common->precision != QCD_PREC_FP64 && common->precision != QCD_PREC_FP32) return QCD_ERR_INVALID;
   if (common->n_or < 0 || common->renorm_every < 0 || common->upd < 0) return QCD_ERR_INVALID;
-  if (common->algo == QCD_ALGO_METROPOLIS && !(common->epsilon > 0.f && common->epsilon < 1.f)) return QCD_ERR_INVALID;
+  if (common->algo == QCD_ALGO_METROPOLIS && !(common->epsilon > 0.f && common->epsilon < 1.f))
+    return QCD_ERR_INVALID;
   qcd_batch* b = new (std::nothrow) qcd_batch();
   if (!b) return QCD_ERR_NOMEM;
   b->common = *common;
@@ -779,7 +782,8 @@ int qcd_batch_autotune(qcd_batch* b, int sweeps_per_trial, long long* bytes_out,
     BCUDA(b, cudaMemcpyAsync(sv.acc, b->accept, (size_t)b->sites * sizeof(int), cudaMemcpyDeviceToDevice, b->stream));
   }
   BCUDA(b, cudaMalloc(&sv.draw, b->n * sizeof(unsigned long long)));
-  BCUDA(b, cudaMemcpyAsync(sv.draw, b->draw_dev, b->n * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, b->stream));
+  BCUDA(b, cudaMemcpyAsync(sv.draw, b->draw_dev, b->n * sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
+                           b->stream));
   BCUDA(b, cudaMalloc(&sv.cur, b->n * sizeof(int)));
   BCUDA(b, cudaMemcpyAsync(sv.cur, b->cursor, b->n * sizeof(int), cudaMemcpyDeviceToDevice, b->stream));
   if (serb) {

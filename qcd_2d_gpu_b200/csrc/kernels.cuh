@@ -145,7 +145,8 @@ __device__ __forceinline__ void aos_stage(double* sh, int slot, const double* __
   }
 }
 template <int N>
-__device__ __forceinline__ void aos_unstage(const double* sh, int slot, double* __restrict__ aos, size_t first, int n) {
+__device__ __forceinline__ void aos_unstage(const double* sh, int slot, double* __restrict__ aos, size_t first,
+                                            int n) {
 #pragma unroll
   for (int k = 0; k < N * 12 / kBlock; k++) {
     const int i = k * kBlock + threadIdx.x;

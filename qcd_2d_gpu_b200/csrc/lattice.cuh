@@ -142,12 +142,15 @@ __host__ __forceinline__ dim3 tile_grid(const Geo& g) {  // Lt and Lx are even
 // never, the set-up is exposed again at the large sizes.  Passes without and
 // with the chain: 16^3 FP64 40 -> 25 us, 24x20x28 28 -> 17, 54x62x70 39 -> 30,
 // 128^3 FP32 over-relaxation 103 -> 90, heat-bath 149 -> 133.
-__device__ __forceinline__ void chain_wait(unsigned int& x) { asm volatile("griddepcontrol.wait;" : "+r"(x)::"memory"); }
+__device__ __forceinline__ void chain_wait(unsigned int& x) {
+  asm volatile("griddepcontrol.wait;" : "+r"(x)::"memory");
+}
 __device__ __forceinline__ void chain_wait(int& x) { asm volatile("griddepcontrol.wait;" : "+r"(x)::"memory"); }
 __device__ __forceinline__ void chain_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>
-__host__ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int block, cudaStream_t stream, A... args) {
+__host__ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int block, cudaStream_t stream,
+                                           A... args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = dim3((unsigned int)block);

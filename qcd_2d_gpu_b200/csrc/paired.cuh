@@ -4,8 +4,8 @@
 // sublattice site id (t < Lt/2, lane 0) and site id + V/4 (t + Lt/2, lane 1)
 // of the same plane share one 32-B record
 //     (w0, w1, x0, x1) (y0, y1, z0, z1)
-// (measured faster than a lo and a hi half-plane per class), so one thread updates both sites with packed two-lane FP32 arithmetic
-// (fma.rn.f32x2 through __ffma2_rn): a quaternion product is 8 packed
+// (measured faster than a lo and a hi half-plane per class), so one thread updates
+// both sites with packed two-lane FP32 arithmetic (fma.rn.f32x2 through __ffma2_rn): a quaternion product is 8 packed
 // multiply-adds for two sites instead of 16 per site, and the neighbour
 // offsets are worked out once for the pair.  Lt/2 is even, so both sites of
 // a pair have the same q = ((t + x) mod 2) xor parity and therefore the same
@@ -128,13 +128,7 @@ struct Pair32 {
   // the pair a thread rewrites
   __device__ __forceinline__ Q2 ld_own(int dir, int par, int j) const { return ld_pair_cg(at(dir, par, j)); }
   __device__ __forceinline__ void st(int dir, int par, int j, const Q2& u) const { st_pair(at(dir, par, j), u); }
-  // one site, by its sublattice index (the one-off kernels: starts, layout changes)
-  __device__ __forceinline__ Quat<float> ld_site(int dir, int par, int id) const {
-    const int lane = id >= vhp, j = id - lane * vhp;
-    const float* lo = reinterpret_cast<const float*>(at(dir, par, j));
-    const float* hi = reinterpret_cast<const float*>(at(dir, par, j) + 1);
-    return Quat<float>{lo[lane], lo[2 + lane], hi[lane], hi[2 + lane]};
-  }
+  // one site, by its sublattice index (the starts)
   __device__ __forceinline__ void st_site(int dir, int par, int id, const Quat<float>& u) const {
     const int lane = id >= vhp, j = id - lane * vhp;
     float* lo = reinterpret_cast<float*>(at(dir, par, j));
@@ -389,8 +383,8 @@ static __global__ void __launch_bounds__(kBlock) normalize32p(Pair32 P) {
 }
 
 // unitarity (kernels.cuh): thread per pair
-static __global__ void __launch_bounds__(kBlock) unitarity_p(Pair32 P, double tol, double2* partials, unsigned int* counter,
-                                                      double* out, const int* err) {
+static __global__ void __launch_bounds__(kBlock) unitarity_p(Pair32 P, double tol, double2* partials,
+                                                             unsigned int* counter, double* out, const int* err) {
   const int j = blockIdx.x * kBlock + threadIdx.x;
   double s = 0, bad = 0;
   if (j < P.vhp) {

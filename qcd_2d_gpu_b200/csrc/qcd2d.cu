@@ -199,10 +199,15 @@ Phase32pFn phase_fn32p(int k, int bc, int kind) {
   }
 }
 
+PhaseArgs phase_args(const qcd_lattice* h, int renorm = 0) {
+  return PhaseArgs{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, renorm,
+                   h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
+}
+
 // one pass over the six phases with one update kind; with `renorm` (FP32
 // only) every link is re-projected as it is stored
 int pass(qcd_lattice* h, int kind, int renorm = 0) {
-  PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, renorm, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
+  PhaseArgs a = phase_args(h, renorm);
   const dim3 grid = tile_grid(h->g), grid_p = tile_grid(h->gh);
   for (int k = 0; k < 6; k++) {
     count_slots(a, h->draw_dev, h->draw_dev + 1, k, kind != KIND_OR);
@@ -443,7 +448,7 @@ int launch_wave(qcd_lattice* h, const PassSpec* ps, int np, int stall_test = 0,
   CUDA_OR_FAIL(h, cudaMemsetAsync(h->wave_done, 0, (size_t)h->g.lt * sizeof(unsigned int), h->stream));
   CUDA_OR_FAIL(h, cudaMemsetAsync(h->wave_queue, 0, sizeof(unsigned int), h->stream));
   CUDA_OR_FAIL(h, cudaMemsetAsync(h->wave_abort, 0, sizeof(int), h->stream));
-  PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, 0, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
+  PhaseArgs a = phase_args(h);
   const int sk = h->p.algo == QCD_ALGO_HEATBATH ? KIND_HB : KIND_METRO;
   const int bc = h->p.boundary;
   const unsigned int grid = (unsigned int)h->wave_grid;
@@ -520,13 +525,14 @@ cudaError_t launch_resident(const qcd_lattice* h, S L, typename S::Global global
   int clusters = 0;
   cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_bytes<S>(kResidentLog));
+    e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             resident_bytes<S>(kResidentLog));
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, (const void*)fn, &c);
   return e != cudaSuccess ? e : clusters > 0 ? cudaSuccess : cudaErrorNotSupported;
 }
 
 cudaError_t resident_call(const qcd_lattice* h, const ResidentProgram& p, bool probe) {
-  PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, 0, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
+  PhaseArgs a = phase_args(h);
   if (h->paired) return launch_resident(h, ClusterPair{{}, h->gh.vh}, pair32(h), h->gh, a, p, probe);
   if (h->p.precision == QCD_PREC_FP64) return launch_resident(h, Cluster64{}, links64(h), h->g, a, p, probe);
   return launch_resident(h, Cluster32{}, links32(h), h->g, a, p, probe);
@@ -590,10 +596,11 @@ int pairs_setup(qcd_lattice* h) {
 // writing the other one, which then becomes current.
 int pass_pairs(qcd_lattice* h, int kind, int renorm) {
   if (!h->q32alt || !h->sms) return fail(h, QCD_ERR_INVALID, "fused pairs used before their setup");
-  PhaseArgs a{h->p.beta, h->p.epsilon, h->p.upd, h->err, h->accept, renorm, h->draw_key, h->draw_dev, 0, 0, philox_keys(h->draw_key)};
+  PhaseArgs a = phase_args(h, renorm);
   const PairMaps& mc = h->pair_maps[h->q32 == h->pair_buf[0] ? 0 : 1];
   const PairMaps& ma = h->pair_maps[h->q32 == h->pair_buf[0] ? 1 : 0];
-  CUDA_OR_FAIL(h, pair_pass32(h->q32, h->q32alt, mc, ma, h->g, h->p.boundary, kind, a, h->pair_seg, h->sms, h->stream));
+  CUDA_OR_FAIL(h, pair_pass32(h->q32, h->q32alt, mc, ma, h->g, h->p.boundary, kind, a, h->pair_seg, h->sms,
+                              h->stream));
   float4* t = h->q32;
   h->q32 = h->q32alt;
   h->q32alt = t;
@@ -644,31 +651,18 @@ int reduce_result(qcd_lattice* h, double* a, double* b) {
 // `err`: the device error word where out_dev has room for it (finish_sum2), or null
 int launch_measure(qcd_lattice* h, double* out_dev, const int* err) {
   const bool pmc = h->p.boundary == QCD_BC_PMC;
-  if (h->p.precision == QCD_PREC_FP64) {
-    const unsigned int nb = measure_blocks(h->g.vh, kMeasurePerSM64);
-    if (pmc)
-      CUDA_OR_FAIL(h, launch_chained(measure<Links64, 1, kMeasurePerSM64>, nb, kBlock, h->stream, links64(h), h->g, h->partials,
-                                     h->counter, out_dev, err));
-    else
-      CUDA_OR_FAIL(h, launch_chained(measure<Links64, 0, kMeasurePerSM64>, nb, kBlock, h->stream, links64(h), h->g, h->partials,
-                                     h->counter, out_dev, err));
-  } else if (h->paired) {
-    const unsigned int nb = measure_blocks(h->gh.vh, kMeasurePerSMPair);
-    if (pmc)
-      CUDA_OR_FAIL(h, launch_chained(measure_p<1>, nb, kBlock, h->stream, pair32(h), h->gh, h->partials,
-                                     h->counter, out_dev, err));
-    else
-      CUDA_OR_FAIL(h, launch_chained(measure_p<0>, nb, kBlock, h->stream, pair32(h), h->gh, h->partials,
-                                     h->counter, out_dev, err));
-  } else {
-    const unsigned int nb = measure_blocks(h->g.vh, kMeasurePerSM32);
-    if (pmc)
-      CUDA_OR_FAIL(h, launch_chained(measure<Links32, 1, kMeasurePerSM32>, nb, kBlock, h->stream, links32(h), h->g, h->partials,
-                                     h->counter, out_dev, err));
-    else
-      CUDA_OR_FAIL(h, launch_chained(measure<Links32, 0, kMeasurePerSM32>, nb, kBlock, h->stream, links32(h), h->g, h->partials,
-                                     h->counter, out_dev, err));
-  }
+  auto launch = [&](auto kernel, auto links, const Geo& g, int per_sm) {
+    return launch_chained(kernel, measure_blocks(g.vh, per_sm), kBlock, h->stream, links, g, h->partials, h->counter,
+                          out_dev, err);
+  };
+  if (h->p.precision == QCD_PREC_FP64)
+    CUDA_OR_FAIL(h, launch(pmc ? measure<Links64, 1, kMeasurePerSM64> : measure<Links64, 0, kMeasurePerSM64>,
+                           links64(h), h->g, kMeasurePerSM64));
+  else if (h->paired)
+    CUDA_OR_FAIL(h, launch(pmc ? measure_p<1> : measure_p<0>, pair32(h), h->gh, kMeasurePerSMPair));
+  else
+    CUDA_OR_FAIL(h, launch(pmc ? measure<Links32, 1, kMeasurePerSM32> : measure<Links32, 0, kMeasurePerSM32>,
+                           links32(h), h->g, kMeasurePerSM32));
   return QCD_OK;
 }
 
@@ -833,7 +827,8 @@ int qcd_create(const qcd_params* p, qcd_lattice** out) {
   if (rc == QCD_OK) step(cudaMalloc(&h->draw_dev, 2 * sizeof(unsigned long long)), "cudaMalloc(draw counter)");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->draw_dev, 0, sizeof(unsigned long long), h->stream), "memset");
   if (rc == QCD_OK) step(cudaMallocHost(&h->result_host, 4 * sizeof(double)), "cudaMallocHost");
-  if (rc == QCD_OK) step(cudaHostGetDevicePointer((void**)&h->result_dev, h->result_host, 0), "cudaHostGetDevicePointer");
+  if (rc == QCD_OK)
+    step(cudaHostGetDevicePointer((void**)&h->result_dev, h->result_host, 0), "cudaHostGetDevicePointer");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->counter, 0, sizeof(unsigned int), h->stream), "memset");
   if (rc == QCD_OK) step(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "memset");
   // the FP64 sweep draws from the stored MRG32k3a streams at every update; an
@@ -1176,13 +1171,14 @@ int qcd_autotune(qcd_lattice* h, int sweeps_per_trial, qcd_tuning* chosen) {
   CUDA_OR_FAIL(h, cudaMemcpyAsync(links_save, lp, lb, cudaMemcpyDeviceToDevice, h->stream));
   if (rng_save) CUDA_OR_FAIL(h, cudaMemcpyAsync(rng_save, h->rng, rng_bytes, cudaMemcpyDeviceToDevice, h->stream));
   if (acc_save)
-    CUDA_OR_FAIL(h, cudaMemcpyAsync(acc_save, h->accept, (size_t)h->V * sizeof(int), cudaMemcpyDeviceToDevice, h->stream));
+    CUDA_OR_FAIL(h, cudaMemcpyAsync(acc_save, h->accept, (size_t)h->V * sizeof(int), cudaMemcpyDeviceToDevice,
+                                    h->stream));
   const long long passes_save = h->unit_passes, sweeps_save = h->sweeps_done;
   unsigned long long draws_save = 0;
   CUDA_OR_FAIL(h, cudaMemcpyAsync(&draws_save, h->draw_dev, sizeof(draws_save), cudaMemcpyDeviceToHost, h->stream));
   CUDA_OR_FAIL(h, cudaStreamSynchronize(h->stream));
-  const int sched_save = h->sched, chunk_save = h->wave_chunk, chain_save = h->wave_chain, fronts_save = h->wave_fronts,
-            pseg_save = h->pair_seg;
+  const int sched_save = h->sched, chunk_save = h->wave_chunk, chain_save = h->wave_chain,
+            fronts_save = h->wave_fronts, pseg_save = h->pair_seg;
   const bool paired_save = h->paired;  // the saved links are in this layout
   cudaEvent_t &e0 = bk.e0, &e1 = bk.e1;
   CUDA_OR_FAIL(h, cudaEventCreate(&e0));
@@ -1332,7 +1328,8 @@ int qcd_check_unitarity(qcd_lattice* h, double tol, double* mean_det) {
   if (h->p.precision == QCD_PREC_FP64)
     unitarity<<<nb, kBlock, 0, h->stream>>>(links64(h), h->g.vh, tol, h->partials, h->counter, h->result_dev, h->err);
   else if (h->paired)
-    unitarity_p<<<nblocks(h->gh.vh), kBlock, 0, h->stream>>>(pair32(h), tol, h->partials, h->counter, h->result_dev, h->err);
+    unitarity_p<<<nblocks(h->gh.vh), kBlock, 0, h->stream>>>(pair32(h), tol, h->partials, h->counter, h->result_dev,
+                                                             h->err);
   else
     unitarity<<<nb, kBlock, 0, h->stream>>>(links32(h), h->g.vh, tol, h->partials, h->counter, h->result_dev, h->err);
   LAUNCH_CHECK(h);
@@ -1499,7 +1496,8 @@ extern "C" int qcd_measure_aos_noalloc(const double* phi_dev, int lt, int lx, in
     return QCD_ERR_UNSUPPORTED;
   }
   const long long vh = (long long)lt * lx * ly / 2;
-  if (measure_blocks(vh, kMeasurePerSM64) > QCD_NOALLOC_MAX_BLOCKS) return QCD_ERR_UNSUPPORTED;  // excluded by the static_assert
+  if (measure_blocks(vh, kMeasurePerSM64) > QCD_NOALLOC_MAX_BLOCKS)  // excluded by the static_assert
+    return QCD_ERR_UNSUPPORTED;
   void* base = nullptr;
   int rc = noalloc_scratch(&base);
   if (rc) return rc;

@@ -11,11 +11,11 @@
 // same order, so the results are theirs.  No wait on memory needs a bound: the
 // CTAs of a cluster run together by construction.
 //
-// What is left is the latency of one update (8^3 takes 2.0 us a phase in FP64, 16^3
+// What is left is the latency of one update (8^3 takes 1.9 us a phase in FP64, 16^3
 // 2.4) and, as the CTAs fill, the rate of remote shared-memory reads, so the whole
-// GPU wins early (resident_items).  Five FP64 heat-bath sweeps of 16^3 95 -> 73 us,
-// of 8^3 95 -> 59 us; two FP32 sweeps with three over-relaxation passes of 16^3
-// 59 -> 39 us, of 18x20x22 61 -> 43 us (chained phase launches -> resident).
+// GPU wins early (kResidentItems).  Phase launches -> cluster, back to back: five FP64
+// heat-bath sweeps of 16^3 88-93 -> 73 us, of 8^3 75 -> 57 us; two FP32 sweeps with three
+// over-relaxation passes of 16^3 110 -> 70 us, of 18x20x22 112 -> 80 us.
 #pragma once
 #include "paired.cuh"
 
@@ -24,12 +24,21 @@ namespace qcd {
 constexpr int kResidentCtas = 16;
 constexpr int kResidentLog = 8;  // most slots of a CTA: 2^8, one thread each
 constexpr int kResidentPasses = 64;
-// Largest work of a phase (sites; pairs) for which one cluster is faster than launches
-// on the whole GPU: heat-bath and over-relaxation 4096 (4000 FP64 sites: five
-// heat-bath sweeps 97 against 100 us; 3360 pairs: 24 phases 64 against 64-77 us,
-// 2048 pairs 44 against 60), Metropolis, whose hits are longer, 2048 (3360 pairs: 218
-// against 205 us) but on single-precision planes, whose sites have half the bytes to
-// fetch (3960 sites: level).
+// Largest work of a phase (sites; pairs) that one cluster takes instead of launches on
+// the whole GPU.  Heat-bath and over-relaxation 4096, phase launches against cluster, us:
+//   2048 pairs   one heat-bath sweep 20.4 / 18.3, two sweeps with three OR passes 123 / 86
+//   2400 pairs                       21.0 / 24.0                                 128 / 122
+//   3360 pairs                       21.5 / 24.8                                 134 / 127
+//   4080 pairs                       21.4 / 25.8                                 132 / 135
+//   2048 FP64    one heat-bath sweep 18.9 / 17.2, five 93 / 75, two with one OR pass 61 / 49
+//   2560 FP64                        20.1 / 21.5       99 / 94                       67 / 61
+//   4000 FP64                        19.8 / 23.1       97 / 101                      66 / 67
+//   4000 planes  one heat-bath sweep 16.1 / 15.8, two with three OR passes 112 / 79
+// so from 2048 to 4096 pairs or FP64 sites the cluster gains where over-relaxation passes
+// or several sweeps share a call, and a call of one sweep is up to a fifth longer.
+// Metropolis, whose hits are longer, 2048 (two sweeps, 2048 FP64 sites 36 / 31, 2048 pairs
+// 46 / 37; 3360 pairs, more hits, 205 / 218) but on single-precision planes, whose sites
+// have half the bytes to fetch (4000 sites 34 / 31).
 constexpr int kResidentItems = 4096, kResidentItemsMetro = 2048;
 static_assert(kResidentItems <= kResidentCtas << kResidentLog, "slots for every site");
 
@@ -139,11 +148,13 @@ struct ClusterPair {
 
 // One staple added to the sum, forward or backward (add_staples, add_staples2)
 template <class R>
-__device__ __forceinline__ Quat<R> add_forward(const Quat<R>& A, const Quat<R>& a, const Quat<R>& b, const Quat<R>& c) {
+__device__ __forceinline__ Quat<R> add_forward(const Quat<R>& A, const Quat<R>& a, const Quat<R>& b,
+                                               const Quat<R>& c) {
   return q_acc_mul_bd(A, q_mul_bd(a, b), c);
 }
 template <class R>
-__device__ __forceinline__ Quat<R> add_backward(const Quat<R>& A, const Quat<R>& a, const Quat<R>& b, const Quat<R>& c) {
+__device__ __forceinline__ Quat<R> add_backward(const Quat<R>& A, const Quat<R>& a, const Quat<R>& b,
+                                                const Quat<R>& c) {
   return q_acc_mul(A, q_mul_adbd(a, b), c);
 }
 __device__ __forceinline__ Q2 add_forward(const Q2& A, const Q2& a, const Q2& b, const Q2& c) {
@@ -224,8 +235,8 @@ __device__ __forceinline__ void resident_update(const Cluster32& L, uint32_t* rn
   L.st(mu, par, n.id, link_new32<KIND>(L, A, g, a, mu, par, n.id, n.id, rn, true));
 }
 template <int KIND>
-__device__ __forceinline__ void resident_update(const ClusterPair& L, uint32_t* rng, const Geo& gh, const PhaseArgs& a,
-                                                const Nbr& n, int mu, int par, int bc, int rn) {
+__device__ __forceinline__ void resident_update(const ClusterPair& L, uint32_t* rng, const Geo& gh,
+                                                const PhaseArgs& a, const Nbr& n, int mu, int par, int bc, int rn) {
   const Q2 A = resident_staples(L, gh, n, mu, par, bc, true);
   L.st(mu, par, n.id, pair_new<KIND>(L, A, a, mu, par, n.id, rn));
 }

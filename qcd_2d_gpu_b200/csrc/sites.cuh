@@ -33,11 +33,12 @@ struct PhaseArgs {
   unsigned int count_add = 0;
 };
 
-// The drawing-phase counter lives on the device as two words, both holding the
-// count between passes; the first is the one that is saved and restored.  A
-// drawing pass advances it without a launch of its own (2 us each before): phases
-// 0-2 read word 0 while phase 0 writes the advanced count to word 1, phases 3-5
-// read word 1 while phase 3 copies it back, so no launch writes the word it reads.
+// The drawing-phase counter lives on the device as word 0, with word 1 as scratch that
+// holds nothing between passes (starts, checkpoints, the other schedules and the cluster
+// set word 0 alone).  A drawing pass advances it without a launch of its own (2 us each
+// before): phases 0-2 read word 0 while phase 0 writes the advanced count to word 1,
+// phases 3-5 read word 1 while phase 3 copies it back, so no launch writes the word it
+// reads.
 template <class Args>
 __host__ inline void count_slots(Args& a, unsigned long long* word0, unsigned long long* word1, int k, bool draws) {
   a.phase_ptr = k < 3 ? word0 : word1;
@@ -248,14 +249,14 @@ __device__ __forceinline__ double plaq(const L& links, int mu, int nu, int p, in
 //
 // Bound by HBM on a large lattice, by the latency of one turn on a small one.
 // A small lattice gets a CTA per 128 indices, one turn each, as long as that
-// leaves SMs idle (16^3: 7 us; with eight sites in series per thread 14 us);
+// leaves SMs idle (16^3: 5 us; with eight sites in series per thread 14 us);
 // above, four turns per CTA, which amortise its reduction where other launches
 // fill the GPU (a batch of 96 replicas: 3% of its run).  A large one gets the CTAs that are
 // resident at once on 148 SMs at the kernel's register count, which then walk
 // the lattice side by side, so neighbours meet in L1 and L2 and no last wave
-// runs half empty.  384^3: FP64 0.95 ms at 2 CTAs per SM (1.26 ms with twice as
-// many CTAs, 1.7 ms with a CTA per 1024 indices and one parity after the other),
-// FP32 0.55 ms at 4, site pairs 0.48 ms at 3 (0.89 ms before).
+// runs half empty.  384^3, thermalised links: FP64 0.95 ms at 2 CTAs per SM (1.26 ms
+// with twice as many CTAs, 1.7 ms with a CTA per 1024 indices and one parity after the
+// other), FP32 0.55 ms at 4, site pairs 0.50-0.60 ms at 3 (0.89 ms before).
 constexpr int kMeasureIds = kBlock / 2;
 constexpr int kMeasureSMs = 148;
 constexpr int kMeasurePerSM64 = 2, kMeasurePerSM32 = 4, kMeasurePerSMPair = 3;

@@ -25,9 +25,11 @@ enum { KIND_METRO = 0, KIND_HB = 1, KIND_OR = 2 };
 // (DEVERR_TIMEOUT: a bounded wait of the wavefront or the fused-pair kernels ran out)
 enum { DEVERR_HB_LOOP = 1, DEVERR_NONUNITARY = 2, DEVERR_TIMEOUT = 4 };
 
-// The Kennedy-Pendleton rejection loop accepts with probability > 1/2 for any
-// staple; this bound is only reached when the staple sum is zero or not
-// finite, and then the update stops and flags the error instead of spinning.
+// The Kennedy-Pendleton rejection loop accepts a try with probability > 1/2 where
+// beta |A| exceeds 1 (|A|: norm of the staple sum, up to 4) and with 0.443 (2 beta
+// |A|)^1.5 where that is small.  This bound is reached when the staple sum is zero or not
+// finite, or with couplings of a few hundredths and less; the update then stops and
+// flags the error instead of spinning.
 #define QCD_HB_MAX_TRIES 4096
 
 template <int MU>
@@ -39,7 +41,8 @@ struct Planes {
 // FP32 staples add their second product straight into the sum with
 // multiply-adds (A + X Y^+, A + X Y); FP64 keeps the reference's separate
 // product and sum, whose rounding the bit-parity tests pin.
-__device__ __forceinline__ Quat<float> q_acc_mul_bd(const Quat<float>& A, const Quat<float>& a, const Quat<float>& b) {
+__device__ __forceinline__ Quat<float> q_acc_mul_bd(const Quat<float>& A, const Quat<float>& a,
+                                                    const Quat<float>& b) {
   Quat<float> c;
   c.w = A.w + a.w * b.w + a.x * b.x + a.y * b.y + a.z * b.z;
   c.x = A.x + a.x * b.w - a.w * b.x - a.y * b.z + a.z * b.y;
@@ -59,7 +62,8 @@ __device__ __forceinline__ Quat<double> q_acc_mul_bd(const Quat<double>& A, cons
                                                      const Quat<double>& b) {
   return q_add(A, q_mul_bd(a, b));
 }
-__device__ __forceinline__ Quat<double> q_acc_mul(const Quat<double>& A, const Quat<double>& a, const Quat<double>& b) {
+__device__ __forceinline__ Quat<double> q_acc_mul(const Quat<double>& A, const Quat<double>& a,
+                                                  const Quat<double>& b) {
   return q_add(A, q_mul(a, b));
 }
 
@@ -190,10 +194,9 @@ __device__ __forceinline__ Quat<double> overrelax_ref(Quat<double> A, const Quat
 //
 // The phase is bound by instruction issue, so the steps are written out short:
 // exact one-step forms of the draws (PhiloxStream::u24), hardware log, sin and
-// cos without the handling of denormals their arguments never are (the
-// results are __logf's, __cosf's and __sincosf's on all 2^24 draws), and the
+// cos without the handling of denormals that their arguments never are, and the
 // accept test in double only where single precision cannot decide it.
-__device__ __forceinline__ float log2_normal(float x) {  // __logf(x) = ln 2 log2_normal(x)
+__device__ __forceinline__ float log2_normal(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
