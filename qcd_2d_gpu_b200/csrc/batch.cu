@@ -325,7 +325,9 @@ struct qcd_batch {
 
 namespace {
 
+// (clears the runtime's record of a failed call: no later call reports it again)
 int bfail(qcd_batch* b, int code, const char* fmt, ...) {
+  if (code == QCD_ERR_CUDA || code == QCD_ERR_NOMEM) cudaGetLastError();
   if (b) {
     va_list ap;
     va_start(ap, fmt);
@@ -338,11 +340,9 @@ int bfail(qcd_batch* b, int code, const char* fmt, ...) {
 #define BCUDA(b, call)                                                                              \
   do {                                                                                              \
     cudaError_t e_ = (call);                                                                        \
-    if (e_ != cudaSuccess) {                                                                        \
-      cudaGetLastError();                                                                           \
+    if (e_ != cudaSuccess)                                                                          \
       return bfail(b, e_ == cudaErrorMemoryAllocation ? QCD_ERR_NOMEM : QCD_ERR_CUDA, "%s: %s", #call, \
                    cudaGetErrorString(e_));                                                         \
-    }                                                                                               \
   } while (0)
 
 // every replica (setup, whole-batch launches)
@@ -721,7 +721,10 @@ int qcd_batch_run(qcd_batch* b, int sweeps, int measure_every, int use_graph) {
       cudaStreamWaitEvent(main, b->join_ev[k], 0);
     }
   }
-  if (rc) return rc;
+  if (rc) {
+    cudaGetLastError();  // (joining the lanes of a failed run may fail too)
+    return rc;
+  }
   b->sweeps_done += sweeps;
   return QCD_OK;
 }

@@ -85,7 +85,10 @@ struct qcd_lattice {
 
 namespace {
 
+// The runtime's record of a failed call is cleared with its report: no later call, of
+// this lattice or another, reports it again.
 int fail(qcd_lattice* h, int code, const char* fmt, ...) {
+  if (code == QCD_ERR_CUDA || code == QCD_ERR_NOMEM) cudaGetLastError();
   if (h) {
     va_list ap;
     va_start(ap, fmt);
@@ -95,12 +98,10 @@ int fail(qcd_lattice* h, int code, const char* fmt, ...) {
   return code;
 }
 
-// (the runtime's record of the error is cleared: a later call must not report it again)
 #define CUDA_OR_FAIL(h, call)                                                                 \
   do {                                                                                        \
     cudaError_t e_ = (call);                                                                  \
     if (e_ != cudaSuccess) {                                                                  \
-      cudaGetLastError();                                                                     \
       if (e_ == cudaErrorMemoryAllocation)                                                    \
         return fail(h, QCD_ERR_NOMEM, "%s: %s", #call, cudaGetErrorString(e_));               \
       return fail(h, QCD_ERR_CUDA, "%s (%s:%d): %s", #call, __FILE__, __LINE__,               \
@@ -398,10 +399,7 @@ int wave_task_table(qcd_lattice* h, int np, const WaveSched& S, int fronts, cons
   if (e == cudaSuccess)
     e = cudaMemcpy(h->wave_tasks[np], host, (size_t)S.n_tasks * sizeof(unsigned int), cudaMemcpyHostToDevice);
   free(host);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(h, QCD_ERR_CUDA, "wavefront task table: %s", cudaGetErrorString(e));
-  }
+  if (e != cudaSuccess) return fail(h, QCD_ERR_CUDA, "wavefront task table: %s", cudaGetErrorString(e));
   h->wave_tasks_chunk[np] = S.chunk_sites;
   h->wave_tasks_fronts[np] = fronts;
   *out = h->wave_tasks[np];
@@ -1212,7 +1210,10 @@ int qcd_autotune(qcd_lattice* h, int sweeps_per_trial, qcd_tuning* chosen) {
   h->wave_chain = chain_save;
   h->wave_fronts = fronts_save;
   h->pair_seg = pseg_save;
-  if (rc) return rc;
+  if (rc) {
+    cudaGetLastError();
+    return rc;
+  }
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune_cache.push_back(TuneChoice{key, cand[best]});
@@ -1413,6 +1414,7 @@ int qcd_rng_tape(unsigned long long seed, long long first, int n_streams, int n_
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpy(host_out, d, n * sizeof(TapeRec), cudaMemcpyDeviceToHost);
   cudaFree(d);
+  if (e != cudaSuccess) cudaGetLastError();
   return e == cudaSuccess ? QCD_OK : QCD_ERR_CUDA;
 }
 
