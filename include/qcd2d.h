@@ -261,8 +261,9 @@ long long qcd_volume(const qcd_lattice* h);
 int qcd_get_params(const qcd_lattice* h, qcd_params* out);
 /* Device pointer and byte size of the current link store (diagnostics,
    benchmarks).  Under QCD_SCHED_PAIRS each pass moves the links to the other
-   of two stores, so the pointer holds until the next sweep.  An FP32 store
-   is in site pairs when qcd_get_pair_layout says so. */
+   of two stores, so the pointer holds until the next sweep.  Six planes, one
+   per direction (y, x, t) and parity, of V/2 links (w, x, y, z) each; an FP32
+   store is in site pairs when qcd_get_pair_layout says so. */
 int qcd_link_store(const qcd_lattice* h, void** dev_ptr, size_t* bytes);
 
 const char* qcd_last_error(const qcd_lattice* h);
